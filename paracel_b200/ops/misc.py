@@ -28,20 +28,21 @@ class RunningTopK:
         self.idx = torch.full((m, k), -1, dtype=torch.int64, device=row_ids.device)
 
     def update(self, S: torch.Tensor, col_ids: torch.Tensor):
-        _lib.check_cuda(S, torch.float32, "S")
+        if not S.is_cuda or S.dtype != torch.float32 or S.dim() != 2 or (S.shape[1] > 1 and S.stride(1) != 1):
+            raise ValueError("S must be a CUDA float32 matrix with contiguous rows")
         _lib.call("pcl_topk_rows", S, S.stride(0), S.shape[0], S.shape[1], self.row_ids,
                   col_ids.to(torch.int64).contiguous(), self.lower, self.k, self.val, self.idx,
                   _lib.stream_ptr())
 
     def result(self):
-        """{row id: [(col id, value), ...]} best first, without empty slots."""
-        out = {}
-        v, i, r = self.val.cpu(), self.idx.cpu(), self.row_ids.cpu()
-        for a in range(r.numel()):
-            lst = [(int(i[a, j]), float(v[a, j])) for j in range(self.k) if int(i[a, j]) >= 0]
-            if lst:
-                out[int(r[a])] = lst
-        return out
+        """{row id: [(col id, value), ...]} best first, without empty slots.  The three tensors become
+        lists in one conversion each (a read of one tensor element costs over a microsecond: 12,007
+        rows x 20 took 1.38 s element by element); the empty slots of a row are its last ones."""
+        filled = (self.idx >= 0).sum(1).tolist()
+        v, i, r = self.val.tolist(), self.idx.tolist(), self.row_ids.tolist()
+        k = self.k
+        return {a: list(zip(ii, vv)) if n == k else list(zip(ii[:n], vv[:n]))
+                for a, ii, vv, n in zip(r, i, v, filled) if n}
 
 
 def gram(H: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:

@@ -146,6 +146,29 @@ def test_running_topk_and_gram():
     torch.testing.assert_close(G.double(), H.double().T @ H.double(), rtol=1e-4, atol=1e-2)
 
 
+@pytest.mark.parametrize("n,pitch,k", [(1, 1, 1), (127, 127, 5), (128, 128, 32), (129, 132, 20), (511, 513, 7),
+                                       (512, 512, 20), (513, 516, 20), (2051, 2052, 32), (1000, 1003, 1)])
+def test_topk_rows_edges_and_ties_match_a_stable_sort(n, pitch, k):
+    """Both row layouts (pitch a multiple of four floats or not) at the edges of the 128- and
+    512-column steps.  Values are small integers, so most are tied: of equal values the earlier
+    column wins, which a stable descending sort gives exactly; each row's own id is left out."""
+    from paracel_b200.ops.misc import RunningTopK
+    g = torch.Generator(device="cuda").manual_seed(n + pitch + k)
+    m = 37
+    S = torch.empty(m, pitch, device="cuda")[:, :n]
+    S.copy_(torch.randint(-9, 10, (m, n), device="cuda", generator=g).float())
+    col_ids = torch.arange(n, device="cuda") + 5
+    row_ids = torch.arange(m, device="cuda") * 3
+    tk = RunningTopK(row_ids, k, lower=-8.0)
+    tk.update(S, col_ids)
+    Sm = torch.where((col_ids[None, :] == row_ids[:, None]) | (S < -8.0), torch.full_like(S, -1e30), S)
+    val, pos = torch.sort(Sm, dim=1, descending=True, stable=True)
+    got = tk.result()
+    for r in range(m):
+        exp = [(int(col_ids[j]), float(x)) for x, j in zip(val[r, :k], pos[r, :k]) if x > -1e29]
+        assert got.get(int(row_ids[r]), []) == exp
+
+
 def test_device_allreduce_single_rank():
     from paracel_b200.ops.misc import DeviceAllReduce
     ar = DeviceAllReduce(device="cuda:0")
