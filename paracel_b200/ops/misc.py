@@ -35,14 +35,11 @@ class RunningTopK:
                   _lib.stream_ptr())
 
     def result(self):
-        """{row id: [(col id, value), ...]} best first, without empty slots.  The three tensors become
-        lists in one conversion each (a read of one tensor element costs over a microsecond: 12,007
-        rows x 20 took 1.38 s element by element); the empty slots of a row are its last ones."""
-        filled = (self.idx >= 0).sum(1).tolist()
-        v, i, r = self.val.tolist(), self.idx.tolist(), self.row_ids.tolist()
-        k = self.k
-        return {a: list(zip(ii, vv)) if n == k else list(zip(ii[:n], vv[:n]))
-                for a, ii, vv, n in zip(r, i, v, filled) if n}
+        """{row id: [(col id, value), ...]} best first, without empty slots.  Built natively from host
+        copies of the three tensors: a read of one tensor element costs over a microsecond (12,007 rows
+        x 20 took 1.38 s element by element)."""
+        from .._core import core
+        return core().topk_lists(self.row_ids.cpu().numpy(), self.idx.cpu().numpy(), self.val.cpu().numpy())
 
 
 def gram(H: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:

@@ -307,3 +307,15 @@ def test_rating_balance_over_the_rank_grid():
             share = torch.bincount(r[i == 0], minlength=npx * npy).double() / cnt
             assert share.max() / share.min() < 1.3
     assert int((balanced_groups(cu, 1) != 0).sum()) == 0
+
+
+@pytest.mark.parametrize("m,k", [(1, 1), (5, 3), (40, 20)])
+def test_topk_lists_ends_a_row_at_its_first_empty_slot(m, k):
+    rng = np.random.default_rng(m * k)
+    ids, val = np.arange(m) * 7, rng.standard_normal((m, k)).astype(np.float32)
+    idx = rng.integers(0, 1 << 40, (m, k))
+    n = rng.integers(0, k + 1, m)
+    for r in range(m):
+        idx[r, n[r]:] = -1
+    exp = {int(ids[r]): [(int(idx[r, j]), float(val[r, j])) for j in range(n[r])] for r in range(m) if n[r]}
+    assert core().topk_lists(ids, idx, val) == exp
