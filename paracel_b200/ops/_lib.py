@@ -66,8 +66,8 @@ SIGS = {
     "pcl_partition_count": "ppqiipp",
     "pcl_partition_scatter": "pppqiipqppppip",
     "pcl_gram": "pqipp",
-    "pcl_spmm_csr": "pppqpipp",
-    "pcl_spmm_csr_t": "pppqpipp",
+    "pcl_spmm_csr": "pppqqpipp",
+    "pcl_spmm_csr_t": "pppqqpipp",
     "pcl_chol_factor": "pippdpp",
     "pcl_allreduce_sum_f64": "ppipppiiiqQpp",
     "pcl_ssp_commit": "piiqpp",

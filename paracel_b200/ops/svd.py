@@ -17,7 +17,7 @@ def spmm_csr(row_ptr: torch.Tensor, cols: torch.Tensor, vals: Optional[torch.Ten
     n, K = row_ptr.numel() - 1, H.shape[1]
     if out is None:
         out = torch.empty(n, K, device=H.device)
-    _lib.call("pcl_spmm_csr", row_ptr, cols, vals, n, H, K, out, _lib.stream_ptr())
+    _lib.call("pcl_spmm_csr", row_ptr, cols, vals, n, cols.numel(), H, K, out, _lib.stream_ptr())
     return out
 
 
@@ -27,7 +27,7 @@ def spmm_csr_t(row_ptr: torch.Tensor, cols: torch.Tensor, vals: Optional[torch.T
     _lib.check_cuda(W, torch.float32, "W")
     _lib.check_cuda(out, torch.float32, "out")
     n, K = row_ptr.numel() - 1, W.shape[1]
-    _lib.call("pcl_spmm_csr_t", row_ptr, cols, vals, n, W, K, out, _lib.stream_ptr())
+    _lib.call("pcl_spmm_csr_t", row_ptr, cols, vals, n, cols.numel(), W, K, out, _lib.stream_ptr())
     return out
 
 

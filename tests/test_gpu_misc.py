@@ -209,3 +209,54 @@ def test_device_balltree_search_matches_host_tree_and_brute_force():
     small.build()
     i2, s2, _ = DeviceBalltree(small).search(queries[:2], 5)
     assert (i2[:, 3:] == -1).all().item() and sorted(i2[0, :3].tolist()) == [0, 1, 2]
+
+
+def _ragged_csr(n, cols, lens, g, weighted=True, lead=0):
+    """CSR with the given row lengths; ``lead`` entries before the first row's."""
+    ptr = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+    ptr[1:] = torch.cumsum(lens, 0)
+    ptr += lead
+    nnz = int(ptr[-1])
+    idx = torch.randint(0, cols, (nnz,), device="cuda", generator=g, dtype=torch.int32)
+    val = torch.randn(nnz, device="cuda", generator=g) if weighted else None
+    return ptr, idx, val
+
+
+@pytest.mark.parametrize("K", [4, 12, 32, 52, 64, 112, 128])
+@pytest.mark.parametrize("shape", ["even", "empty_rows", "one_long_row", "offset_unaligned", "single"])
+def test_csr_products_match_fp64(K, shape):
+    """Both CSR products, cut by entries: rows cut by segment and block boundaries, runs of empty rows
+    longer than a block's row cache, a row far longer than a block, row pointers that do not start at
+    zero, arrays off the 16-byte grid.  A sum of n fp32 products is within n 2^-24 of the sum of
+    their magnitudes."""
+    from paracel_b200.ops.svd import spmm_csr, spmm_csr_t
+    g = torch.Generator(device="cuda").manual_seed(K)
+    n, N, lead = 3001, 501, 0
+    lens = torch.randint(0, 40, (n,), device="cuda", generator=g)
+    if shape == "empty_rows":
+        n = 9000
+        lens = torch.zeros(n, dtype=torch.int64, device="cuda")
+        lens[torch.tensor([0, 5, 6, 3000, 3001, 8990], device="cuda")] = torch.tensor([3, 1, 700, 2, 129, 64], device="cuda")
+    elif shape == "one_long_row":
+        lens[17] = 70_003
+    elif shape == "offset_unaligned":
+        lead = 37
+    elif shape == "single":
+        n, lens = 1, torch.tensor([1], device="cuda")
+    ptr, idx, val = _ragged_csr(n, N, lens, g, weighted=shape != "even", lead=lead)
+    if shape == "offset_unaligned":
+        idx, val, ptr = idx[1:], val[1:], ptr - 1
+    H = torch.randn(N, K, device="cuda", generator=g)
+    W = torch.randn(n, K, device="cuda", generator=g)
+    out = spmm_csr(ptr, idx, val, H)
+    back = torch.ones(N, K, device="cuda")
+    spmm_csr_t(ptr, idx, val, W, back)
+    rows = torch.repeat_interleave(torch.arange(n, device="cuda"), lens)
+    a, b = int(ptr[0]), int(ptr[-1])
+    c, v = idx[a:b].long(), torch.ones(b - a, device="cuda").double() if val is None else val[a:b].double()
+    for got, dst, src, at, start in ((out, rows, H, c, 0.0), (back, c, W, rows, 1.0)):
+        prod = v[:, None] * src.double()[at]
+        ref = torch.full(got.shape, start, dtype=torch.float64, device="cuda").index_add_(0, dst, prod)
+        mag = torch.full(got.shape, start, dtype=torch.float64, device="cuda").index_add_(0, dst, prod.abs())
+        cnt = torch.bincount(dst, minlength=got.shape[0]).double()[:, None] + 2
+        assert bool(((got.double() - ref).abs() <= cnt * 2.0 ** -24 * mag).all())
