@@ -59,7 +59,7 @@ SIGS = {
     "pcl_pagerank_pull_stream": "ppppqqppfpppppip",
     "pcl_lda_gibbs": "ppppppqifffQip",
     "pcl_lda_loglik": "ppppppqifffpp",
-    "pcl_als_solve": "pppppppppppqifip",
+    "pcl_als_solve": "ppppppppppqqiiifp",
     "pcl_kmeans_accumulate": "ppqippp",
     "pcl_topk_rows": "pqiippfippp",
     "pcl_balltree_search": "pppppppiiipppp",

@@ -25,24 +25,20 @@ def als_solve(user_ptr: torch.Tensor, item_idx: torch.Tensor, rating: torch.Tens
     _lib.validate_ids(item_idx.contiguous(), 0, H.shape[0], "ALS ratings (item rows)")
     K = _kpad(k)
     W = torch.zeros(n_users, k, device=dev)
-    cnt = (user_ptr[1:] - user_ptr[:-1])
-    nseg = torch.clamp((cnt + seg_len - 1) // seg_len, min=1)
-    nseg = torch.where(cnt > 0, nseg, torch.zeros_like(nseg))
-    total = int(nseg.sum().item())
-    if total == 0:
+    nnz = item_idx.numel()
+    if n_users <= 0 or nnz == 0:
         return W
-    seg_user = torch.repeat_interleave(torch.arange(n_users, device=dev), nseg)
-    first = torch.cumsum(nseg, 0) - nseg
-    within = torch.arange(total, device=dev) - first[seg_user]
-    seg_begin = user_ptr[:-1][seg_user] + within * seg_len
-    seg_end = torch.minimum(seg_begin + seg_len, user_ptr[1:][seg_user])
-    split = nseg > 1
-    n_slots = int(split.sum().item())
-    slot = torch.full((n_users,), -1, dtype=torch.int32, device=dev)
-    slot[split] = torch.arange(n_slots, dtype=torch.int32, device=dev)
-    scratch = torch.zeros(max(n_slots, 1) * (K * K + K), device=dev)
-    counts = torch.zeros(max(n_slots, 1), dtype=torch.int32, device=dev)
-    _lib.call("pcl_als_solve", seg_user.int().contiguous(), seg_begin.contiguous(), seg_end.contiguous(),
-              nseg.int().contiguous(), slot, item_idx.int().contiguous(), rating.float().contiguous(), H, W,
-              scratch, counts, total, k, float(lam), 0, _lib.stream_ptr())
+    # At most 2048 users are split, which bounds the scratch (135 MB at rank 128) without asking the
+    # device how many there are; a split user's pieces are a quarter as long, so that the last ones
+    # to run are short.
+    split = max(int(seg_len), (nnz + 2047) // 2048)
+    piece = max(split // 4, 256)
+    slots = nnz // split + 1
+    seg_cap = n_users + nnz // piece + slots
+    scratch = torch.empty(slots * (K * K + K), device=dev)
+    ints = torch.empty(slots + 8 + 3 * seg_cap + 4 * n_users, dtype=torch.int32, device=dev)
+    slot_count, counters, seg, lists = ints.split([slots, 8, 3 * seg_cap, 4 * n_users])
+    _lib.call("pcl_als_solve", user_ptr.long().contiguous(), item_idx.int().contiguous(),
+              rating.float().contiguous(), H, W, scratch, slot_count, counters, seg, lists, n_users, split, piece,
+              seg_cap, k, float(lam), _lib.stream_ptr())
     return W

@@ -260,3 +260,33 @@ def test_csr_products_match_fp64(K, shape):
         mag = torch.full(got.shape, start, dtype=torch.float64, device="cuda").index_add_(0, dst, prod.abs())
         cnt = torch.bincount(dst, minlength=got.shape[0]).double()[:, None] + 2
         assert bool(((got.double() - ref).abs() <= cnt * 2.0 ** -24 * mag).all())
+
+
+@pytest.mark.parametrize("k", [7, 18, 33, 50, 65, 100, 128])
+def test_als_forms_match_fp64_at_their_edges(k):
+    """Users on both sides of every form's limits (warp / CTA dual form, k x k form, split users)."""
+    from paracel_b200.ops.als import als_solve
+    g = torch.Generator(device="cuda").manual_seed(k)
+    ni, lam = 700, 0.5
+    cnt = [0, 1, 2, 15, 16, 17, 31, 32, 33, 63, 64, 65, 95, 96, 97, 128, 129, 300, 511, 512, 0, 1024, 1025, 2700, 3]
+    cnt += [c for c in (k - 1, k, k + 1)]
+    ptr = torch.tensor([0] + cnt).cumsum(0).cuda() + 5          # the arrays begin before the first user
+    H = torch.randn(ni, k, device="cuda", generator=g)
+    idx = torch.randint(0, ni, (int(ptr[-1]),), device="cuda", generator=g).int()
+    r = torch.randn(int(ptr[-1]), device="cuda", generator=g)
+    W = als_solve(ptr, idx, r, H, lam, seg_len=1024)
+    W0 = als_solve(ptr, idx, r, H, 0.0, seg_len=1024)           # without lambda: the k x k form only
+    for u, c in enumerate(cnt):
+        a, b = int(ptr[u]), int(ptr[u + 1])
+        Hs, rs = H[idx[a:b].long()].double(), r[a:b].double()
+        if c == 0:
+            assert not bool(W[u].any()) and not bool(W0[u].any())
+            continue
+        for got, l in ((W[u], lam), (W0[u], 0.0)):
+            G = Hs.T @ Hs + l * torch.eye(k, device="cuda").double()
+            if l == 0.0 and c < 2 * k:
+                continue                                        # singular or nearly so
+            ref = torch.linalg.solve(G, Hs.T @ rs)
+            # backward error of the Gram sums and of the factorisation, both in fp32
+            bound = 16 * 2.0 ** -24 * float(torch.linalg.cond(G)) * float(ref.norm())
+            assert float((got.double() - ref).norm()) <= bound, (u, c, l)
