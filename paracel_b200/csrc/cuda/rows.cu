@@ -235,7 +235,9 @@ __global__ void scalars_push_kernel(ScalarArgs a) {
   }
 }
 
-// int32 rows (LDA word-topic counts): pull = copy, push = integer add of deltas.
+// int32 rows (LDA word-topic counts): pull = copy, push = integer add of deltas.  A warp takes a row;
+// IU 16-byte pieces per lane are in flight before the first is stored or reduced.
+constexpr int IU = 4;
 struct IRowArgs {
   const long long* ids;
   int* const* shards;
@@ -248,7 +250,12 @@ struct IRowArgs {
   long long rows;
   PclStatus* status;
   int rank;
+  int vec;  // push: cur and old start on 16-byte boundaries
 };
+
+__device__ __forceinline__ int4 ld_int4(const int* p, int vec) {
+  return vec ? *reinterpret_cast<const int4*>(p) : make_int4(p[0], p[1], p[2], p[3]);
+}
 
 __global__ void __launch_bounds__(256) irows_pull_kernel(IRowArgs a) {
   const int vec_per_row = a.D >> 2;
@@ -261,19 +268,28 @@ __global__ void __launch_bounds__(256) irows_pull_kernel(IRowArgs a) {
       continue;
     }
     const int* src = a.shards[(int)(g % a.world)] + (g / a.world) * a.D;
-    for (int v = lane; v < vec_per_row; v += 32) {
-      int4 x;
-      asm volatile("ld.relaxed.sys.global.v4.s32 {%0,%1,%2,%3}, [%4];"
-                   : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w)
-                   : "l"(src + 4 * v));
-      *reinterpret_cast<int4*>(a.cur + row * a.D + 4 * v) = x;
-      if (a.old) *reinterpret_cast<int4*>(a.old + row * a.D + 4 * v) = x;
+    for (int v0 = lane; v0 < vec_per_row; v0 += 32 * IU) {
+      int4 x[IU];
+#pragma unroll
+      for (int u = 0; u < IU; ++u)
+        if (v0 + 32 * u < vec_per_row)
+          asm volatile("ld.relaxed.sys.global.v4.s32 {%0,%1,%2,%3}, [%4];"
+                       : "=r"(x[u].x), "=r"(x[u].y), "=r"(x[u].z), "=r"(x[u].w)
+                       : "l"(src + 4 * (v0 + 32 * u)));
+#pragma unroll
+      for (int u = 0; u < IU; ++u) {
+        if (v0 + 32 * u >= vec_per_row) continue;
+        const long long at = row * a.D + 4 * (v0 + 32 * u);
+        *reinterpret_cast<int4*>(a.cur + at) = x[u];
+        if (a.old) *reinterpret_cast<int4*>(a.old + at) = x[u];
+      }
     }
   }
 }
 
 __global__ void __launch_bounds__(256) irows_push_kernel(IRowArgs a) {
   if (pcl_status_code(a.status) != 0) return;
+  const int vec_per_row = a.D >> 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
   for (long long row = (long long)blockIdx.x * wpb + warp; row < a.n;
        row += (long long)gridDim.x * wpb) {
@@ -283,18 +299,36 @@ __global__ void __launch_bounds__(256) irows_push_kernel(IRowArgs a) {
       continue;
     }
     int* dstp = a.shards[(int)(g % a.world)] + (g / a.world) * a.D;
-    for (int e = lane; e < a.D; e += 32) {
-      int x = a.cur[row * a.D + e];
-      int d = a.old ? x - a.old[row * a.D + e] : x;
-      if (d != 0)
-        asm volatile("red.relaxed.sys.global.add.s32 [%0], %1;" ::"l"(dstp + e), "r"(d)
-                     : "memory");
+    const int* c = a.cur + row * a.D;
+    const int* o = a.old ? a.old + row * a.D : nullptr;
+    for (int v0 = lane; v0 < vec_per_row; v0 += 32 * IU) {
+      int4 x[IU], y[IU];
+#pragma unroll
+      for (int u = 0; u < IU; ++u) {
+        const int v = v0 + 32 * u;
+        x[u] = v < vec_per_row ? ld_int4(c + 4 * v, a.vec) : make_int4(0, 0, 0, 0);
+        y[u] = o && v < vec_per_row ? ld_int4(o + 4 * v, a.vec) : make_int4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (int u = 0; u < IU; ++u) {
+        int* p = dstp + 4 * (v0 + 32 * u);
+        const int d[4] = {x[u].x - y[u].x, x[u].y - y[u].y, x[u].z - y[u].z, x[u].w - y[u].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (d[e] != 0)
+            asm volatile("red.relaxed.sys.global.add.s32 [%0], %1;" ::"l"(p + e), "r"(d[e]) : "memory");
+      }
     }
   }
   if (a.old != nullptr && a.refresh_old) {   // second sweep, see rows_push_kernel
     for (long long row = (long long)blockIdx.x * wpb + warp; row < a.n;
          row += (long long)gridDim.x * wpb)
-      for (int e = lane; e < a.D; e += 32) a.old[row * a.D + e] = a.cur[row * a.D + e];
+      for (int v = lane; v < vec_per_row; v += 32) {
+        const int4 x = ld_int4(a.cur + row * a.D + 4 * v, a.vec);
+        int* o = a.old + row * a.D + 4 * v;
+        if (a.vec) *reinterpret_cast<int4*>(o) = x;
+        else { o[0] = x.x; o[1] = x.y; o[2] = x.z; o[3] = x.w; }
+      }
   }
 }
 
@@ -361,7 +395,7 @@ PCL_API int pcl_rows_pull_i32(const long long* ids, int* const* shards, int worl
                               int rank, cudaStream_t stream) {
   if (D <= 0 || (D & 3)) return (int)cudaErrorInvalidValue;
   if (n <= 0) return 0;
-  IRowArgs a{ids, shards, world, D, n, cur, old, 0, rows, status, rank};
+  IRowArgs a{ids, shards, world, D, n, cur, old, 0, rows, status, rank, 1};
   irows_pull_kernel<<<grid_for(n, 8, 148 * 16), 256, 0, stream>>>(a);
   return pcl_last_error();
 }
@@ -371,7 +405,8 @@ PCL_API int pcl_rows_push_i32(const long long* ids, int* const* shards, int worl
                               PclStatus* status, int rank, cudaStream_t stream) {
   if (D <= 0 || (D & 3)) return (int)cudaErrorInvalidValue;
   if (n <= 0) return 0;
-  IRowArgs a{ids, shards, world, D, n, cur, old, refresh_old, rows, status, rank};
+  const int vec = ((reinterpret_cast<uintptr_t>(cur) | reinterpret_cast<uintptr_t>(old)) & 15) == 0;
+  IRowArgs a{ids, shards, world, D, n, cur, old, refresh_old, rows, status, rank, vec};
   irows_push_kernel<<<grid_for(n, 8, 148 * 16), 256, 0, stream>>>(a);
   return pcl_last_error();
 }

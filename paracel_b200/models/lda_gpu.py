@@ -131,8 +131,10 @@ class LdaGibbsGpu(paralg):
                 _lib.call("pcl_lda_loglik", bt["ptr"], bt["widx"], self.n_dk[bt["d0"]:bt["d1"]], cur,
                           self.nk_cur, self.doc_len[bt["d0"]:bt["d1"]], nd, self.K, self.alpha, self.beta,
                           self.V * self.beta, self.ll, s)
-            self.paracel_bupdate_multi(bt["keys"], cur, "", "gLDA_word_update", old=old)
-            self.paracel_bupdate_multi(self.k_ts, self.nk_cur, "", "gLDA_sum_topic_update", old=self.nk_old)
+            # the next step pulls both copies anew, so `old` is not brought up to date here
+            self.paracel_bupdate_multi(bt["keys"], cur, "", "gLDA_word_update", old=old, refresh_old=False)
+            self.paracel_bupdate_multi(self.k_ts, self.nk_cur, "", "gLDA_sum_topic_update", old=self.nk_old,
+                                       refresh_old=False)
         elif self._dev_wait_needed(self.clock - self.limit_s):
             self.dev_clock.wait()
         self.iter_commit()

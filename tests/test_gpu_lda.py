@@ -75,3 +75,26 @@ def test_lda_gpu_other_topic_counts(K):
     assert torch.equal(torch.bincount(m.z.long(), minlength=K).int(), m.ts.shard[0].int())
     assert ll[-1] > ll[0]
     m.free()
+
+
+@pytest.mark.parametrize("K", [128, 192, 512, 1024])
+def test_lda_loglik_matches_fp64(K):
+    """Documents of no, one, two and three tokens (a warp takes two at a time); 192: the general kernel."""
+    from paracel_b200.ops import _lib
+    g = torch.Generator(device="cuda").manual_seed(K)
+    lens = torch.tensor([0, 1, 2, 3, 40, 0, 7] * 30, device="cuda")
+    ptr = torch.zeros(lens.numel() + 1, dtype=torch.int64, device="cuda")
+    ptr[1:] = lens.cumsum(0)
+    V, alpha, beta, T = 50, 0.1, 0.01, int(lens.sum())
+    words = torch.randint(0, V, (T,), device="cuda", generator=g).int()
+    n_dk = torch.randint(0, 4, (lens.numel(), K), device="cuda", generator=g).int()
+    n_wk = torch.randint(-1, 9, (V, K), device="cuda", generator=g).int()
+    n_k = torch.randint(50, 900, (K,), device="cuda", generator=g).int()
+    out = torch.zeros(1, dtype=torch.float64, device="cuda")
+    _lib.call("pcl_lda_loglik", ptr, words, n_dk, n_wk, n_k, lens.int(), lens.numel(), K, alpha, beta, V * beta, out,
+              _lib.stream_ptr())
+    doc = torch.repeat_interleave(torch.arange(lens.numel(), device="cuda"), lens)
+    th = (n_dk.double() + alpha) / (lens.double()[:, None] + K * alpha) / (n_k.double() + V * beta)
+    ref = torch.log((th[doc] * (n_wk.double().clamp(min=0) + beta)[words.long()]).sum(1)).sum()
+    # positive terms: a relative error of a few roundings per token, and of the fast logarithm
+    assert abs(float(out) - float(ref)) <= T * (K / 32 + 16) * 2.0 ** -24 + 2e-6 * abs(float(ref))

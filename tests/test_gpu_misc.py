@@ -290,3 +290,36 @@ def test_als_forms_match_fp64_at_their_edges(k):
             # backward error of the Gram sums and of the factorisation, both in fp32
             bound = 16 * 2.0 ** -24 * float(torch.linalg.cond(G)) * float(ref.norm())
             assert float((got.double() - ref).norm()) <= bound, (u, c, l)
+
+
+@pytest.mark.parametrize("width", [4, 124, 128, 132, 1024])
+@pytest.mark.parametrize("lead", [0, 1])
+def test_int_row_table_pull_push_match_torch(width, lead):
+    """Widths around a warp's 128 columns and its four pieces in flight; buffers off 16-byte boundaries."""
+    from paracel_b200.ps.tables import RowTable
+    g = torch.Generator(device="cuda").manual_seed(width)
+    rows, n = 301, 207
+    t = RowTable(rows, width, dtype=torch.int32, device="cuda:0")
+    t.shard.copy_(torch.randint(-99, 99, (rows, width), device="cuda", generator=g))
+    ids = torch.randperm(rows, device="cuda", generator=g)[:n]
+    before = t.shard.clone()
+    cur, old = (torch.zeros(n, width, dtype=torch.int32, device="cuda") for _ in range(2))
+    t.pull(ids, cur, old)
+    assert torch.equal(cur, before[ids]) and torch.equal(old, cur)
+    new = (cur + torch.randint(-2, 3, cur.shape, device="cuda", generator=g)).int()
+
+    def shifted(x):
+        b = torch.zeros(x.numel() + 4, dtype=torch.int32, device="cuda")[lead: lead + x.numel()]
+        return b.copy_(x.reshape(-1)).view(x.shape)
+    new, old = shifted(new), shifted(old)
+    t.push(ids, new, old, refresh_old=False)
+    exp = before.clone()
+    exp[ids] = new
+    assert torch.equal(t.shard, exp) and torch.equal(old, cur)
+    t.push(ids, new, old)                      # the same difference again, and old brought up to date
+    exp[ids] += new - cur
+    assert torch.equal(t.shard, exp) and torch.equal(old, new)
+    t.push(ids, new)
+    exp[ids] += new
+    assert torch.equal(t.shard, exp)
+    t.free()
