@@ -4,6 +4,8 @@
 //
 //   spmm_csr      out[r, :]  = sum_j A[r, c_j] * H[c_j, :]      (K <= 128)
 //   spmm_csr_t    out[c, :] += A[r, c] * W[r, :]                (vector reductions, fp32)
+//   rows_times    out = M P, or (M P) P^T, for tall M and a small square P (K <= 112)
+//   mt19937       the start matrix: U(0, 1) of the host generator of the same seed
 //   chol_factor   G = L L^T for a small K x K Gram matrix; writes R = L^T and T = L^-T so that
 //                 Q = M T is orthonormal and M = Q R, and G^-1 = T T^T.  One CTA, fp64 in
 //                 shared memory.  A pivot below the tolerance marks the matrix rank deficient in
@@ -178,6 +180,126 @@ int launch_spmm(const long long* row_ptr, const int* cols, const float* vals, lo
   return pcl_last_error();
 }
 
+// out = M P (TWICE: (M P) P^T) for M [n x K] and P [K x K], K a multiple of 4, fp32 throughout.  A
+// block of 256 threads takes 64 rows at a time: thread (ty, tx) owns rows 4 ty .. 4 ty + 3 and columns
+// tx + 16 j; P and, for the second product, its transpose stay in shared memory, and the product of
+// the first takes the place of the rows there.  Bound by shared-memory loads (4 + 4 KB per 16 KB
+// multiply-adds) at K = 32, where M itself comes out of L2.
+template <int KB, bool TWICE>
+__global__ void __launch_bounds__(256) rows_times_kernel(const float* __restrict__ M, long long n, int K,
+                                                         const float* __restrict__ P, float* __restrict__ out) {
+  constexpr int N = 16 * KB;             // columns, padded with zeros
+  extern __shared__ __align__(16) float sm[];
+  const int LM = K + 4;
+  float* sP = sm;                        // K x N
+  float* sQ = sP + (TWICE ? K * N : 0);  // K x N: P^T
+  float* sM = sQ + K * N;                // 64 x LM
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  for (int e = tid; e < K * N; e += 256) {
+    const int q = e / N, c = e % N;
+    sP[e] = c < K ? __ldg(P + q * K + c) : 0.f;
+    if (TWICE) sQ[e] = c < K ? __ldg(P + c * K + q) : 0.f;
+  }
+  const int K4 = K / 4;
+  for (long long r0 = (long long)blockIdx.x * 64; r0 < n; r0 += (long long)gridDim.x * 64) {
+    __syncthreads();
+    for (int e = tid; e < 64 * K4; e += 256) {
+      const int r = e / K4, c = 4 * (e % K4);
+      *reinterpret_cast<float4*>(sM + r * LM + c) =
+          r0 + r < n ? __ldg(reinterpret_cast<const float4*>(M + (r0 + r) * K + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int pass = 0; pass < (TWICE ? 2 : 1); ++pass) {
+      const float* B = pass == 0 ? sP : sQ;
+      float acc[4][KB];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < KB; ++j) acc[i][j] = 0.f;
+#pragma unroll 2
+      for (int q = 0; q < K; q += 4) {
+        float4 m[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) m[i] = *reinterpret_cast<const float4*>(sM + (4 * ty + i) * LM + q);
+#pragma unroll
+        for (int j = 0; j < KB; ++j) {
+          const float* b = B + q * N + tx + 16 * j;
+          const float b0 = b[0], b1 = b[N], b2 = b[2 * N], b3 = b[3 * N];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            acc[i][j] = fmaf(m[i].x, b0, acc[i][j]);
+            acc[i][j] = fmaf(m[i].y, b1, acc[i][j]);
+            acc[i][j] = fmaf(m[i].z, b2, acc[i][j]);
+            acc[i][j] = fmaf(m[i].w, b3, acc[i][j]);
+          }
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < KB; ++j)
+          if (tx + 16 * j < K) sM[(4 * ty + i) * LM + tx + 16 * j] = acc[i][j];
+      __syncthreads();
+    }
+    for (int e = tid; e < 64 * K4; e += 256) {
+      const int r = e / K4, c = 4 * (e % K4);
+      if (r0 + r < n)
+        *reinterpret_cast<float4*>(out + (r0 + r) * K + c) = *reinterpret_cast<const float4*>(sM + r * LM + c);
+    }
+  }
+}
+
+template <int KB, bool TWICE>
+int launch_rows_times(const float* M, long long n, int K, const float* P, float* out, cudaStream_t stream) {
+  const size_t smem = ((size_t)K * 16 * KB * (TWICE ? 2 : 1) + 64 * (size_t)(K + 4)) * sizeof(float);
+  cudaError_t e = cudaFuncSetAttribute(rows_times_kernel<KB, TWICE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  int per_sm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rows_times_kernel<KB, TWICE>, 256, smem);
+  if (e != cudaSuccess) return (int)e;
+  long long blocks = (n + 63) / 64;
+  const long long most = 148LL * (per_sm > 0 ? per_sm : 1);
+  if (blocks > most) blocks = most;
+  rows_times_kernel<KB, TWICE><<<(int)blocks, 256, smem, stream>>>(M, n, K, P, out);
+  return pcl_last_error();
+}
+
+// out[i] = scale * u_i + shift with u_i = (word_i mod 2^24) / 2^24 for the words of the Mersenne Twister
+// MT19937 (Matsumoto and Nishimura, 1998) after init_genrand(seed): the stream of the host
+// generator, made where it is used.
+// One block: 227 words of the recurrence are independent of one another, so a step makes 227 and ends
+// with a barrier; tempering and the store are off that chain.
+__global__ void __launch_bounds__(256) mt19937_kernel(float* __restrict__ out, long long n, unsigned seed,
+                                                      float scale, float shift) {
+  __shared__ unsigned x[1024];           // word k at k mod 1024: the last 624 and the 227 in the making
+  const int t = threadIdx.x;
+  if (t == 0) {
+    unsigned s = seed;
+    x[0] = s;
+    for (int k = 1; k < 624; ++k) {
+      s = 1812433253u * (s ^ (s >> 30)) + (unsigned)k;
+      x[k] = s;
+    }
+  }
+  __syncthreads();
+  for (long long i0 = 0; i0 < n; i0 += 227) {
+    if (t < 227) {
+      const int k = (int)((i0 + t) & 1023);
+      const unsigned y = (x[k] & 0x80000000u) | (x[(k + 1) & 1023] & 0x7fffffffu);
+      unsigned v = x[(k + 397) & 1023] ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
+      x[(k + 624) & 1023] = v;
+      v ^= v >> 11;
+      v ^= (v << 7) & 0x9d2c5680u;
+      v ^= (v << 15) & 0xefc60000u;
+      v ^= v >> 18;
+      if (i0 + t < n) out[i0 + t] = fmaf((float)(v & 0xffffffu) * (1.f / 16777216.f), scale, shift);
+    }
+    __syncthreads();
+  }
+}
+
 // One CTA.  Shared memory: L (K x K doubles) and X = L^-1 (K x K doubles).
 __global__ void __launch_bounds__(256) chol_factor_kernel(const float* __restrict__ G, int K,
                                                           float* __restrict__ T, float* __restrict__ R,
@@ -261,6 +383,29 @@ PCL_API int pcl_spmm_csr_t(const long long* row_ptr, const int* cols, const floa
   if (n_rows <= 0 || n_ent <= 0) return 0;
   if (K <= 0 || K > 128 || (K & 3)) return (int)cudaErrorInvalidValue;
   return launch_spmm<true>(row_ptr, cols, vals, n_rows, n_ent, W, K, out, stream);
+}
+
+// M and out 16-byte aligned, K <= 112 a multiple of 4; twice: out = (M P) P^T, else M P.
+PCL_API int pcl_rows_times(const float* M, long long n, int K, const float* P, int twice, float* out,
+                           cudaStream_t stream) {
+  if (n <= 0) return 0;
+  if (K <= 0 || K > 112 || (K & 3)) return (int)cudaErrorInvalidValue;
+#define PCL_RT(KB)                                                                    \
+  case KB:                                                                            \
+    return twice ? launch_rows_times<KB, true>(M, n, K, P, out, stream)               \
+                 : launch_rows_times<KB, false>(M, n, K, P, out, stream);
+  switch ((K + 15) / 16) {
+    PCL_RT(1) PCL_RT(2) PCL_RT(3) PCL_RT(4) PCL_RT(5) PCL_RT(6) PCL_RT(7)
+  }
+#undef PCL_RT
+  return (int)cudaErrorInvalidValue;
+}
+
+PCL_API int pcl_mt19937_uniform(float* out, long long n, unsigned int seed, float scale, float shift,
+                                cudaStream_t stream) {
+  if (n <= 0) return 0;
+  mt19937_kernel<<<1, 256, 0, stream>>>(out, n, seed, scale, shift);
+  return pcl_last_error();
 }
 
 PCL_API int pcl_chol_factor(const float* G, int K, float* T, float* R, double rel_tol, int* info,

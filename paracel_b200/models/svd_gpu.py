@@ -11,18 +11,17 @@ writes its part into ``paracel_delta_buffer(key)`` and a collective ``paracel_bu
 sum.  Stage 2 is the Cholesky-QR of W and H (``M^T M = R^T R``, ``Q = M R^-1``) and the SVD of the
 K x K matrix ``R_W R_H^T`` (on the host, svd.hpp:294-298), ``U = Q_W U_r``, ``V = Q_H V_r``.
 
-Kernels: CSR products ``A.H`` / ``A^T.W`` and the small Cholesky factor (csrc/cuda/svd.cu), the
-Gram matrix (``pcl_gram``), and the tcgen05 GEMM (3xTF32) for the skinny products with K x K
-matrices."""
+Kernels: CSR products ``A.H`` / ``A^T.W`` (the second on a transposed copy of A made by ``load``),
+products of a tall matrix with a K x K one and the small Cholesky factor (csrc/cuda/svd.cu), and the
+Gram matrix (``pcl_gram``)."""
 from __future__ import annotations
 
 import os
 
 import torch
 
-from ..ops.gemm import gemm_nt
 from ..ops.misc import gram
-from ..ops.svd import chol_factor, spmm_csr, spmm_csr_t
+from ..ops.svd import chol_factor, host_rand, rows_times, spmm_csr
 from ..paralg import paralg
 
 
@@ -59,15 +58,30 @@ class SvdGpu(paralg):
         self.vals = vals.to(dev, torch.float32).contiguous()
         _lib.validate_ids(self.cols, 0, self.N, "SVD input (column ids)")
         self.m = self.row_ptr.numel() - 1
+        # A^T in the same form: its products then add up in registers.  Scattering an entry at a time
+        # into A^T W queues up at the popular columns: 1 ms a product on 6.5 M Zipf(1.1) entries,
+        # K = 32, against 0.14 ms for A H.
+        first, last = (int(self.row_ptr[0].item()), int(self.row_ptr[-1].item())) if self.m > 0 else (0, 0)
+        c, order = torch.sort(self.cols[first:last], stable=True)
+        row_of = torch.repeat_interleave(torch.arange(self.m, device=dev, dtype=torch.int32),
+                                         self.row_ptr[1:] - self.row_ptr[:-1])
+        self.t_rows, self.t_vals = row_of[order], self.vals[first:last][order]
+        self.t_ptr = torch.zeros(self.N + 1, dtype=torch.int64, device=dev)
+        self.t_ptr[1:] = torch.cumsum(torch.bincount(c, minlength=self.N), 0)
 
-    def _reduce(self, key: str, part: torch.Tensor) -> torch.Tensor:
-        """Sum of ``part`` over the ranks through the table ``key``: owners start from zero, a
-        collective bupdate adds every rank's part, a read gathers the result."""
+    def _reduce(self, key: str, buf: torch.Tensor, cols: int) -> torch.Tensor:
+        """Sum over the ranks of what each wrote into ``buf``, the delta buffer of the table ``key``:
+        owners start from zero, a collective bupdate adds every rank's part, a read gathers the result."""
         self.paracel_local_shard(key).zero_()
-        buf = self.paracel_delta_buffer(key)
-        buf.copy_(part.reshape(-1))
         self.paracel_bupdate(key, buf, "", self.update_function, collective=True)
-        return self.paracel_read(key).view(part.shape).clone()
+        return self.paracel_read(key).view(-1, cols).clone()
+
+    def _sum_gram(self, W: torch.Tensor) -> torch.Tensor:
+        """``W^T W`` over all ranks."""
+        buf = self.paracel_delta_buffer("WtW").zero_()
+        if self.m:
+            gram(W, buf.view(self.K, self.K))
+        return self._reduce("WtW", buf, self.K)
 
     def _times_inverse(self, M: torch.Tensor, G: torch.Tensor) -> torch.Tensor:
         """``M @ pinv(G)`` for a K x K Gram matrix: ``(M T) T^T`` with the Cholesky factor, or
@@ -78,7 +92,7 @@ class SvdGpu(paralg):
         if info != 0:
             Tf, _ = _orth_fallback(G)
             return (M @ Tf) @ Tf.T
-        return gemm_nt(gemm_nt(M, T.T.contiguous(), precise=True), T, precise=True)
+        return rows_times(M, T, twice=True)
 
     def _orth(self, G: torch.Tensor):
         T, R, info = chol_factor(G, rel_tol=1e-7)
@@ -88,22 +102,22 @@ class SvdGpu(paralg):
 
     def solve(self):
         dev, K, N = self.device, self.K, self.N
-        g = torch.Generator()
-        g.manual_seed(self.seed)
-        H = (torch.rand(N, K, generator=g) * 2 - 1).to(dev)      # same H on every rank
+        H = host_rand((N, K), self.seed, dev, 2.0, -1.0)          # same H on every rank
         A = (self.row_ptr, self.cols, self.vals)
         for _ in range(self.iters):
             W = self._times_inverse(spmm_csr(*A, H), gram(H))
-            WtW = self._reduce("WtW", gram(W) if self.m else torch.zeros(K, K, device=dev))
-            AtW = self._reduce("AtW", spmm_csr_t(*A, W, torch.zeros(N, K, device=dev)))
+            WtW = self._sum_gram(W)
+            buf = self.paracel_delta_buffer("AtW")
+            spmm_csr(self.t_ptr, self.t_rows, self.t_vals, W, buf.view(N, K))
+            AtW = self._reduce("AtW", buf, K)
             H = self._times_inverse(AtW, WtW)
         W = self._times_inverse(spmm_csr(*A, H), gram(H))
-        Tw, Rw = self._orth(self._reduce("WtW", gram(W) if self.m else torch.zeros(K, K, device=dev)))
+        Tw, Rw = self._orth(self._sum_gram(W))
         Th, Rh = self._orth(gram(H))
-        def times(M, T):      # M @ T on the tensor cores when T is square
+        def times(M, T):
             if M.shape[0] == 0 or T.shape[0] != T.shape[1]:
                 return M @ T
-            return gemm_nt(M, T.T.contiguous(), precise=True)
+            return rows_times(M, T)
         Qw, Qh = times(W, Tw), times(H, Th)
         Ur, S, Vrt = torch.linalg.svd((Rw @ Rh.T).double().cpu())      # small K x K problem on the host
         kk = min(self.k, S.numel())

@@ -22,6 +22,7 @@ _LIB_PATH = Path(__file__).resolve().parent.parent / "_lib" / "libpcl_kernels.so
 _T = {
     "p": ctypes.c_void_p,
     "i": ctypes.c_int,
+    "I": ctypes.c_uint,
     "q": ctypes.c_longlong,
     "Q": ctypes.c_ulonglong,
     "f": ctypes.c_float,
@@ -68,6 +69,8 @@ SIGS = {
     "pcl_gram": "pqipp",
     "pcl_spmm_csr": "pppqqpipp",
     "pcl_spmm_csr_t": "pppqqpipp",
+    "pcl_rows_times": "pqipipp",
+    "pcl_mt19937_uniform": "pqIffp",
     "pcl_chol_factor": "pippdpp",
     "pcl_allreduce_sum_f64": "ppipppiiiqQpp",
     "pcl_ssp_commit": "piiqpp",

@@ -1,5 +1,6 @@
 """Wrappers of the device SVD kernels (``csrc/cuda/svd.cu``): CSR x dense products with a
-skinny right-hand side and the Cholesky factor of a small Gram matrix."""
+skinny right-hand side, tall matrices times small square ones, the host generator's stream on the
+device and the Cholesky factor of a small Gram matrix."""
 from __future__ import annotations
 
 from typing import Optional, Tuple
@@ -28,6 +29,29 @@ def spmm_csr_t(row_ptr: torch.Tensor, cols: torch.Tensor, vals: Optional[torch.T
     _lib.check_cuda(out, torch.float32, "out")
     n, K = row_ptr.numel() - 1, W.shape[1]
     _lib.call("pcl_spmm_csr_t", row_ptr, cols, vals, n, cols.numel(), W, K, out, _lib.stream_ptr())
+    return out
+
+
+def rows_times(M: torch.Tensor, P: torch.Tensor, twice: bool = False) -> torch.Tensor:
+    """``M @ P`` or, with ``twice``, ``(M @ P) @ P.T`` for ``M [n, K]`` and ``P [K, K]``, K <= 112 a
+    multiple of 4."""
+    _lib.check_cuda(M, torch.float32, "M")
+    _lib.check_cuda(P, torch.float32, "P")
+    K = M.shape[1]
+    if P.shape != (K, K) or K % 4 or K > 112 or (M.data_ptr() & 15):
+        raise ValueError("P must be K x K for the K <= 112 columns of an aligned M, K a multiple of 4")
+    out = torch.empty_like(M)
+    _lib.call("pcl_rows_times", M, M.shape[0], K, P, int(twice), out, _lib.stream_ptr())
+    return out
+
+
+def host_rand(shape, seed: int, device, scale: float = 1.0, shift: float = 0.0) -> torch.Tensor:
+    """``torch.rand(shape, generator=g) * scale + shift`` for a fresh CPU generator ``g`` with
+    ``manual_seed(seed)``, made on the device (number for number where the scaled values are exact,
+    as they are for 2 and -1)."""
+    out = torch.empty(shape, device=device)
+    _lib.call("pcl_mt19937_uniform", out, out.numel(), int(seed) & 0xffffffff, float(scale), float(shift),
+              _lib.stream_ptr())
     return out
 
 

@@ -323,3 +323,30 @@ def test_int_row_table_pull_push_match_torch(width, lead):
     exp[ids] += new
     assert torch.equal(t.shard, exp)
     t.free()
+
+
+@pytest.mark.parametrize("K", [4, 12, 16, 20, 32, 52, 100, 112])
+def test_rows_times_matches_fp64(K):
+    """Row counts around a block's 64 rows, columns around the 16 of a thread row."""
+    from paracel_b200.ops.svd import rows_times
+    g = torch.Generator(device="cuda").manual_seed(K)
+    P = torch.randn(K, K, device="cuda", generator=g)
+    for n in (1, 63, 64, 65, 20_011):
+        M = torch.randn(n, K, device="cuda", generator=g)
+        A, P64 = M.double().abs() @ P.double().abs(), P.double()
+        u = 2.0 ** -24 * (K + 1)
+        one = rows_times(M, P)
+        assert bool(((one.double() - M.double() @ P64).abs() <= u * A).all())
+        two = rows_times(M, P, twice=True)
+        bound = 2.1 * u * (A @ P64.abs().T)
+        assert bool(((two.double() - M.double() @ P64 @ P64.T).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("n,seed", [(1, 0), (226, 3), (227, 3), (228, 7), (1023, 2 ** 32 - 1), (100_003, -5)])
+def test_host_rand_is_the_cpu_generators_stream(n, seed):
+    from paracel_b200.ops.svd import host_rand
+    g = torch.Generator()
+    g.manual_seed(seed)
+    ref = torch.rand(n, generator=g)
+    assert torch.equal(host_rand((n,), seed, "cuda").cpu(), ref)
+    assert torch.equal(host_rand((n,), seed, "cuda", 2.0, -1.0).cpu(), ref * 2 - 1)
