@@ -8,10 +8,9 @@
 // The accumulated g is what the reference's "dgd" method pushes with one bupdate per
 // round; here it is written straight into the delta vector that dense_bupdate reduces.
 //
-// Dense kernel: one warp per row, theta cached in shared memory, per-block partial
-// gradient in shared memory, then a two-stage reduction through a scratch buffer
-// (blocks x d partials, summed in block order by the last block) so that the result
-// does not depend on atomics between blocks.
+// Dense kernel: a warp per row (or a few rows), per-block partial gradient, then a second
+// kernel adds the blocks x d partials up in a fixed order, so that the result does not
+// depend on atomics between blocks.
 // Sparse kernel: CSR rows, one warp per row; features with index < hot_T (the most
 // frequent ones after frequency renumbering) accumulate in shared memory per block,
 // the others go to global memory with red.add.
@@ -30,89 +29,34 @@ struct DenseGradArgs {
   long long n;
   int d;
   int logistic;
-  float* g;            // d, written (not accumulated)
-  double* loss;        // 1, written
   float* scratch;      // gridDim.x * d partial gradients + gridDim.x loss partials (as 2 floats each)
-  unsigned int* counter;  // zero before the first launch; the last block resets it
   int private_acc;     // 1: every warp owns a d-float accumulator in shared memory (no atomics)
 };
 
 __device__ __forceinline__ float sigmoidf_(float z) { return 1.f / (1.f + __expf(-z)); }
 
-// R > 0: d <= 32 * R, the row and this warp's gradient sums stay in registers (R values per lane,
-// X is read exactly once); R == 0: any d, the row is read twice (the second time from cache).
-template <int R>
-__global__ void __launch_bounds__(256) dense_grad_kernel(DenseGradArgs a) {
-  extern __shared__ float sm[];
-  float* s_theta = sm;          // d
-  float* s_g = sm + a.d;        // d
-  __shared__ double s_loss[8];
-  __shared__ int is_last;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-  for (int j = threadIdx.x; j < a.d; j += blockDim.x) s_theta[j] = a.theta[j];
-  for (int j = threadIdx.x; j < (a.private_acc ? wpb : 1) * a.d; j += blockDim.x) s_g[j] = 0.f;
-  __syncthreads();
-  double loss = 0.0;
-  float gacc[R > 0 ? R : 1];
-#pragma unroll
-  for (int t = 0; t < (R > 0 ? R : 1); ++t) gacc[t] = 0.f;
-  for (long long row = (long long)blockIdx.x * wpb + warp; row < a.n; row += (long long)gridDim.x * wpb) {
-    const float* x = a.X + row * a.d;
-    float xr[R > 0 ? R : 1];
-    float z = 0.f;
-    if constexpr (R > 0) {
-#pragma unroll
-      for (int t = 0; t < R; ++t) {
-        const int j = lane + 32 * t;
-        xr[t] = j < a.d ? __ldg(x + j) : 0.f;
-      }
-#pragma unroll
-      for (int t = 0; t < R; ++t) {
-        const int j = lane + 32 * t;
-        z = fmaf(xr[t], j < a.d ? s_theta[j] : 0.f, z);
-      }
-    } else {
-      for (int j = lane; j < a.d; j += 32) z = fmaf(x[j], s_theta[j], z);
-    }
-    z = pcl_warp_sum(z);
-    const float yy = a.y[row];
-    float r;
-    if (a.logistic) {
-      const float h = sigmoidf_(z);
-      r = yy - h;
-      // log-loss with clamping so that a saturated sigmoid does not give inf
-      const float hc = fminf(fmaxf(h, 1e-7f), 1.f - 1e-7f);
-      loss += (yy == 1.f) ? -(double)__logf(hc) : -(double)__logf(1.f - hc);
-    } else {
-      r = yy - z;
-      loss += (double)r * (double)r;
-    }
-    if constexpr (R > 0) {
-#pragma unroll
-      for (int t = 0; t < R; ++t) gacc[t] = fmaf(r, xr[t], gacc[t]);
-    } else if (a.private_acc) {
-      // entry j of this warp's accumulator is only ever touched by lane j % 32 of this warp
-      float* gw = s_g + (long long)warp * a.d;
-      for (int j = lane; j < a.d; j += 32) gw[j] = fmaf(r, x[j], gw[j]);
-    } else {
-      for (int j = lane; j < a.d; j += 32) atomicAdd(&s_g[j], r * x[j]);
-    }
+// residual of a row from its margin z; adds the row's loss
+__device__ __forceinline__ float dg_residual(const DenseGradArgs& a, float z, float yy, double& loss) {
+  if (a.logistic) {
+    const float h = sigmoidf_(z);
+    // log-loss with clamping so that a saturated sigmoid does not give inf
+    const float hc = fminf(fmaxf(h, 1e-7f), 1.f - 1e-7f);
+    loss += (yy == 1.f) ? -(double)__logf(hc) : -(double)__logf(1.f - hc);
+    return yy - h;
   }
-  if constexpr (R > 0) {   // registers -> this warp's slot in shared memory
-    float* gw = s_g + (long long)warp * a.d;
-#pragma unroll
-    for (int t = 0; t < R; ++t) {
-      const int j = lane + 32 * t;
-      if (j < a.d) gw[j] = gacc[t];
-    }
-  }
-  if (lane == 0) s_loss[warp] = loss;  // identical in every lane of the warp
-  __syncthreads();
+  const float r = yy - z;
+  loss += (double)r * (double)r;
+  return r;
+}
+
+// The block's partial gradient (the slots of its warps in s_g) and loss into the scratch.
+__device__ __forceinline__ void dg_store_partial(const DenseGradArgs& a, const float* s_g, int slots,
+                                                 const double* s_loss) {
+  const int wpb = blockDim.x >> 5;
   float* part = a.scratch + (long long)blockIdx.x * a.d;
   for (int j = threadIdx.x; j < a.d; j += blockDim.x) {
     float v = s_g[j];
-    if (a.private_acc)
-      for (int w = 1; w < wpb; ++w) v += s_g[(long long)w * a.d + j];
+    for (int w = 1; w < slots; ++w) v += s_g[(long long)w * a.d + j];
     part[j] = v;
   }
   if (threadIdx.x == 0) {
@@ -120,26 +64,148 @@ __global__ void __launch_bounds__(256) dense_grad_kernel(DenseGradArgs a) {
     for (int w = 0; w < wpb; ++w) l += s_loss[w];
     reinterpret_cast<double*>(a.scratch + (((long long)gridDim.x * a.d + 1) & ~1LL))[blockIdx.x] = l;
   }
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const unsigned int prev = atomicAdd(a.counter, 1u);
-    is_last = (prev == gridDim.x - 1);
+}
+
+constexpr int dg_blocks_per_sm(int P) { return P >= 4 ? 2 : 4; }
+
+// Rows of up to 128 * P floats: theta, the rows and this warp's gradient sums stay in registers, and
+// X is read exactly once.  A warp takes ROWS rows per step, all their loads in flight before the first
+// is used.  VEC: rows start on 16-byte boundaries (d a multiple of 4) and a lane takes columns
+// 128 t + 4 lane + q; otherwise 128 t + 32 q + lane.
+template <int P, int ROWS, bool VEC>
+__global__ void __launch_bounds__(256, dg_blocks_per_sm(P)) dense_grad_rows_kernel(DenseGradArgs a) {
+  extern __shared__ float s_g[];      // 8 x d
+  __shared__ double s_loss[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+  auto col = [&](int t, int q) { return VEC ? 128 * t + 4 * lane + q : 128 * t + 32 * q + lane; };
+  float th[P][4], gacc[P][4];
+#pragma unroll
+  for (int t = 0; t < P; ++t)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      th[t][q] = col(t, q) < a.d ? __ldg(a.theta + col(t, q)) : 0.f;
+      gacc[t][q] = 0.f;
+    }
+  double loss = 0.0;
+  const long long step = (long long)gridDim.x * wpb * ROWS;
+  for (long long row = ((long long)blockIdx.x * wpb + warp) * ROWS; row < a.n; row += step) {
+    float x[ROWS][P][4], z[ROWS], yy[ROWS];
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+      const bool in = row + k < a.n;
+      const float* xp = a.X + (row + k) * a.d;
+#pragma unroll
+      for (int t = 0; t < P; ++t) {
+        if constexpr (VEC) {
+          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (in && col(t, 0) < a.d) v = __ldg(reinterpret_cast<const float4*>(xp + col(t, 0)));
+          x[k][t][0] = v.x; x[k][t][1] = v.y; x[k][t][2] = v.z; x[k][t][3] = v.w;
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) x[k][t][q] = in && col(t, q) < a.d ? __ldg(xp + col(t, q)) : 0.f;
+        }
+      }
+      yy[k] = in ? __ldg(a.y + row + k) : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+      z[k] = 0.f;
+#pragma unroll
+      for (int t = 0; t < P; ++t)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) z[k] = fmaf(x[k][t][q], th[t][q], z[k]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int k = 0; k < ROWS; ++k) z[k] += __shfl_xor_sync(0xffffffffu, z[k], o);
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+      if (row + k >= a.n) break;
+      const float r = dg_residual(a, z[k], yy[k], loss);
+#pragma unroll
+      for (int t = 0; t < P; ++t)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) gacc[t][q] = fmaf(r, x[k][t][q], gacc[t][q]);
+    }
   }
+#pragma unroll
+  for (int t = 0; t < P; ++t)
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (col(t, q) < a.d) s_g[warp * a.d + col(t, q)] = gacc[t][q];
+  if (lane == 0) s_loss[warp] = loss;  // identical in every lane of the warp
   __syncthreads();
-  if (!is_last) return;
-  __threadfence();
-  for (int j = threadIdx.x; j < a.d; j += blockDim.x) {
-    float s = 0.f;
-    for (unsigned int b = 0; b < gridDim.x; ++b) s += __ldcg(a.scratch + (long long)b * a.d + j);
-    a.g[j] = s;
+  dg_store_partial(a, s_g, wpb, s_loss);
+}
+
+// Any d: the row is read twice (the second time from cache).
+__global__ void __launch_bounds__(256) dense_grad_kernel(DenseGradArgs a) {
+  extern __shared__ float sm[];
+  float* s_theta = sm;          // d
+  float* s_g = sm + a.d;        // d, or 8 x d with private accumulators
+  __shared__ double s_loss[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+  for (int j = threadIdx.x; j < a.d; j += blockDim.x) s_theta[j] = a.theta[j];
+  for (int j = threadIdx.x; j < (a.private_acc ? wpb : 1) * a.d; j += blockDim.x) s_g[j] = 0.f;
+  __syncthreads();
+  double loss = 0.0;
+  for (long long row = (long long)blockIdx.x * wpb + warp; row < a.n; row += (long long)gridDim.x * wpb) {
+    const float* x = a.X + row * a.d;
+    float z = 0.f;
+#pragma unroll 8
+    for (int j = lane; j < a.d; j += 32) z = fmaf(x[j], s_theta[j], z);
+    z = pcl_warp_sum(z);
+    const float r = dg_residual(a, z, a.y[row], loss);
+    if (a.private_acc) {
+      // entry j of this warp's accumulator is only ever touched by lane j % 32 of this warp
+      float* gw = s_g + (long long)warp * a.d;
+#pragma unroll 8
+      for (int j = lane; j < a.d; j += 32) gw[j] = fmaf(r, x[j], gw[j]);
+    } else {
+      for (int j = lane; j < a.d; j += 32) atomicAdd(&s_g[j], r * x[j]);
+    }
   }
-  if (threadIdx.x == 0) {
-    const double* lp = reinterpret_cast<const double*>(a.scratch + (((long long)gridDim.x * a.d + 1) & ~1LL));
+  if (lane == 0) s_loss[warp] = loss;  // identical in every lane of the warp
+  __syncthreads();
+  dg_store_partial(a, s_g, a.private_acc ? wpb : 1, s_loss);
+}
+
+// g[d] and *loss from the `blocks` partials, in a fixed order.  A block owns 32 columns: warp w sums
+// the partials w, w + 8, ..., eight in flight per lane; block 0 sums the losses as well.  (When the
+// last block of the gradient kernel added the partials up one after the other, that chain was most of
+// a step on a small table.)
+__global__ void __launch_bounds__(256) dense_grad_sum_kernel(const float* scratch, int blocks, int d, float* g,
+                                                             double* loss) {
+  __shared__ float s_p[8][32];
+  __shared__ double s_l[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int j = blockIdx.x * 32 + lane;
+  float s = 0.f;
+  if (j < d) {
+#pragma unroll 8
+    for (int b = warp; b < blocks; b += 8) s += __ldg(scratch + (long long)b * d + j);
+  }
+  s_p[warp][lane] = s;
+  if (blockIdx.x == 0) {
+    const double* lp = reinterpret_cast<const double*>(scratch + (((long long)blocks * d + 1) & ~1LL));
     double l = 0.0;
-    for (unsigned int b = 0; b < gridDim.x; ++b) l += __ldcg(lp + b);
-    *a.loss = l;
-    *a.counter = 0u;
+#pragma unroll 4
+    for (int b = threadIdx.x; b < blocks; b += 256) l += __ldg(lp + b);
+    l = pcl_warp_sum_d(l);
+    if (lane == 0) s_l[warp] = l;
+  }
+  __syncthreads();
+  if (warp == 0 && j < d) {
+    float t = s_p[0][lane];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) t += s_p[w][lane];
+    g[j] = t;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    double l = 0.0;
+    for (int w = 0; w < 8; ++w) l += s_l[w];
+    *loss = l;
   }
 }
 
@@ -266,22 +332,40 @@ __global__ void __launch_bounds__(256) sparse_grad_kernel(SparseGradArgs a) {
   if (lane == 0 && loss != 0.0) atomicAdd(a.loss, loss);
 }
 
-template <int R>
-int launch_dense_grad_r(const DenseGradArgs& a, int blocks, size_t smem, cudaStream_t stream) {
-  cudaError_t e = cudaFuncSetAttribute(dense_grad_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
+template <typename F>
+int dg_launch(F kernel, const DenseGradArgs& a, int blocks, size_t smem, cudaStream_t stream) {
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  dense_grad_kernel<R><<<blocks, 256, smem, stream>>>(a);
+  kernel<<<blocks, 256, smem, stream>>>(a);
   return pcl_last_error();
 }
 
-// rows of up to 1024 floats are kept in registers (needs the per-warp shared-memory slots)
-int launch_dense_grad(const DenseGradArgs& a, int blocks, size_t smem, cudaStream_t stream) {
-  if (a.private_acc && a.d <= 128) return launch_dense_grad_r<4>(a, blocks, smem, stream);
-  if (a.private_acc && a.d <= 256) return launch_dense_grad_r<8>(a, blocks, smem, stream);
-  if (a.private_acc && a.d <= 512) return launch_dense_grad_r<16>(a, blocks, smem, stream);
-  if (a.private_acc && a.d <= 1024) return launch_dense_grad_r<32>(a, blocks, smem, stream);
-  return launch_dense_grad_r<0>(a, blocks, smem, stream);
+// The grid: one wave, and at least two steps a warp, since every block costs a row of partials.
+template <int P, int ROWS>
+int dg_launch_rows(const DenseGradArgs& a, int* blocks, cudaStream_t stream) {
+  const long long most = 148LL * dg_blocks_per_sm(P), need = (a.n + 16 * ROWS - 1) / (16 * ROWS);
+  if (*blocks > most) *blocks = (int)most;
+  if (*blocks > need) *blocks = (int)need;
+  const size_t smem = 8 * (size_t)a.d * sizeof(float);
+  if ((a.d & 3) == 0 && (reinterpret_cast<uintptr_t>(a.X) & 15) == 0)
+    return dg_launch(dense_grad_rows_kernel<P, ROWS, true>, a, *blocks, smem, stream);
+  return dg_launch(dense_grad_rows_kernel<P, ROWS, false>, a, *blocks, smem, stream);
+}
+
+// Rows of up to 1024 floats are kept in registers; ROWS puts 16 values per lane in flight (32 from
+// d > 256 on, where fewer warps are resident).
+int launch_dense_grad(DenseGradArgs a, int blocks, float* g, double* loss, cudaStream_t stream) {
+  // per-warp accumulators (8 warps) when they fit into shared memory, else one shared accumulator
+  a.private_acc = (9 * (size_t)a.d * sizeof(float) <= 200 * 1024) ? 1 : 0;
+  int rc;
+  if (a.d <= 128) rc = dg_launch_rows<1, 4>(a, &blocks, stream);
+  else if (a.d <= 256) rc = dg_launch_rows<2, 2>(a, &blocks, stream);
+  else if (a.d <= 512) rc = dg_launch_rows<4, 2>(a, &blocks, stream);
+  else if (a.d <= 1024) rc = dg_launch_rows<8, 1>(a, &blocks, stream);
+  else rc = dg_launch(dense_grad_kernel, a, blocks, (a.private_acc ? 9 : 2) * (size_t)a.d * sizeof(float), stream);
+  if (rc != 0) return rc;
+  dense_grad_sum_kernel<<<(a.d + 31) / 32, 256, 0, stream>>>(a.scratch, blocks, a.d, g, loss);
+  return pcl_last_error();
 }
 
 }  // namespace
@@ -292,21 +376,17 @@ PCL_API long long pcl_lr_dense_scratch_floats(int blocks, int d) {
 }
 
 // g[d] = sum_rows (y - h(theta.x)) x, *loss = summed loss.  `scratch` must hold
-// pcl_lr_dense_scratch_floats(blocks, d) floats (8-byte aligned); `counter` is one
-// zero-initialised unsigned int that the kernel leaves at zero.  d <= 12000.
+// pcl_lr_dense_scratch_floats(blocks, d) floats (8-byte aligned).  d <= 12000.
 PCL_API int pcl_lr_dense_grad(const float* X, const float* y, const float* theta, long long n, int d,
-                              int logistic, float* g, double* loss, float* scratch,
-                              unsigned int* counter, int blocks, cudaStream_t stream) {
+                              int logistic, float* g, double* loss, float* scratch, int blocks,
+                              cudaStream_t stream) {
   if (n <= 0 || d <= 0) return (int)cudaErrorInvalidValue;
   if (d > 12000) return (int)cudaErrorInvalidValue;
   if (blocks <= 0) blocks = 148 * 2;
   long long need = (n + 7) / 8;
   if (need < blocks) blocks = (int)need;
-  // per-warp accumulators (8 warps) when they fit into shared memory, else one shared accumulator
-  const int private_acc = (9 * (size_t)d * sizeof(float) <= 200 * 1024) ? 1 : 0;
-  DenseGradArgs a{X, y, theta, n, d, logistic, g, loss, scratch, counter, private_acc};
-  size_t smem = (private_acc ? 9 : 2) * (size_t)d * sizeof(float);
-  return launch_dense_grad(a, blocks, smem, stream);
+  DenseGradArgs a{X, y, theta, n, d, logistic, scratch, 0};
+  return launch_dense_grad(a, blocks, g, loss, stream);
 }
 
 PCL_API int pcl_lr_sparse_grad(const long long* row_ptr, const int* cols, const float* vals,
@@ -340,19 +420,16 @@ PCL_API int pcl_lr_sparse_grad(const long long* row_ptr, const int* cols, const 
 // that handed all of its HBM to one arena at start-up, a plug-in that runs
 // inside somebody else's memory pool, or a latency-critical loop where the
 // implicit device synchronisation of cudaMalloc/cudaFree is not acceptable.  For
-// them the block partials and the block counter of dense_grad_kernel live in
-// the two file-scope device arrays below instead of a caller-provided scratch
-// tensor.  The price: every GPU that loads this library carries the
+// them the block partials live in the file-scope device array below instead of
+// a caller-provided scratch tensor.  The price: every GPU that loads this library carries the
 // PCL_NOALLOC_MAX_FLOATS * 4 bytes (4 MiB) until the process exits, and all
 // calls on one device share the array, so two calls that overlap on the GPU
 // (different streams) would overwrite each other's partials.
 static __device__ __align__(256) float g_noalloc_scratch[PCL_NOALLOC_MAX_FLOATS];
-static __device__ __align__(256) unsigned int g_noalloc_counter[64];
 
 namespace {
 struct NoAllocSlot {
   float* scratch = nullptr;
-  unsigned int* counter = nullptr;
   bool ready = false;
 };
 NoAllocSlot g_noalloc_slots[64];        // filled under g_noalloc_mutex, one entry per device
@@ -397,8 +474,8 @@ PCL_API int pcl_lr_dense_grad_noalloc(const float* X, const float* y, const floa
   NoAllocSlot& slot = g_noalloc_slots[dev];
   std::lock_guard<std::mutex> guard(g_noalloc_mutex);   // set-up and launch of one call at a time
   if (!slot.ready) {
-    // One-time set-up for this device (it is the current device): translate the symbols
-    // into device addresses.  In host code the array names are only stand-ins.
+    // One-time set-up for this device (it is the current device): translate the symbol
+    // into a device address.  In host code the array name is only a stand-in.
     void* p = nullptr;
     e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
     if (e != cudaSuccess) {
@@ -406,22 +483,11 @@ PCL_API int pcl_lr_dense_grad_noalloc(const float* X, const float* y, const floa
       return (int)e;
     }
     slot.scratch = (float*)p;
-    e = cudaGetSymbolAddress(&p, g_noalloc_counter);
-    if (e != cudaSuccess) {
-      snprintf(g_noalloc_msg, sizeof(g_noalloc_msg), "cudaGetSymbolAddress(counter) failed: %s", cudaGetErrorString(e));
-      return (int)e;
-    }
-    slot.counter = (unsigned int*)p;
     slot.ready = true;
   }
-  // the counter must start at zero whatever an earlier (possibly aborted) call left behind;
-  // the partials are fully overwritten by the kernel before they are read
-  e = cudaMemsetAsync(slot.counter, 0, sizeof(unsigned int), stream);
-  if (e != cudaSuccess) return noalloc_fail(e, "cudaMemsetAsync(counter)");
-  const int private_acc = (9 * (size_t)d * sizeof(float) <= 200 * 1024) ? 1 : 0;   // as pcl_lr_dense_grad
-  DenseGradArgs a{X, y, theta, n, d, logistic, g, loss, slot.scratch, slot.counter, private_acc};
-  size_t smem = (private_acc ? 9 : 2) * (size_t)d * sizeof(float);
-  const int rc = launch_dense_grad(a, blocks, smem, stream);
+  // the partials are fully overwritten by the first kernel before the second reads them
+  DenseGradArgs a{X, y, theta, n, d, logistic, slot.scratch, 0};
+  const int rc = launch_dense_grad(a, blocks, g, loss, stream);
   if (rc != 0) return noalloc_fail((cudaError_t)rc, "kernel launch");
   return 0;
 }

@@ -14,7 +14,7 @@
 //   pcl_lr_dense_grad_noalloc computes exactly what pcl_lr_dense_grad computes
 //   (g[d] = sum over rows of (y - h(theta.x)) * x and the summed loss, h =
 //   sigmoid when `logistic` is non-zero, identity otherwise) but takes no
-//   scratch and no counter argument.
+//   scratch argument.
 //
 // Limits and rules:
 //   * blocks * d + 2 * blocks + 4 must not exceed PCL_NOALLOC_MAX_FLOATS
@@ -26,8 +26,7 @@
 //     (cudaGetSymbolAddress, with that device current).  Make that first call
 //     outside of any stream capture.
 //   * All calls on a device share the array and it keeps what the last call
-//     left there.  The call clears the one word that has to start at zero
-//     itself.  Two calls whose kernels can overlap on the GPU (different
+//     left there.  Two calls whose kernels can overlap on the GPU (different
 //     streams without an ordering between them) race on the array: order them.
 //   * The function calls no cudaMalloc, cudaFree or other allocating routine.
 //     The 4 MiB themselves are taken by the CUDA runtime when it loads this

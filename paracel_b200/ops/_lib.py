@@ -54,7 +54,7 @@ SIGS = {
     "pcl_publish_flag": "piiqp",
     "pcl_dense_push": "ppqqiifp",
     "pcl_validate_ids": "piqqqqpip",
-    "pcl_lr_dense_grad": "pppqiippppip",
+    "pcl_lr_dense_grad": "pppqiipppip",
     "pcl_lr_sparse_grad": "pppppqiippip",
     "pcl_pagerank_pull": "ppppqfppppiqpip",
     "pcl_pagerank_pull_stream": "ppppqqppfpppppip",

@@ -13,7 +13,6 @@ class DenseGrad:
     def __init__(self, d: int, device, blocks: int = 592):
         self.d, self.blocks = d, blocks
         self.scratch = torch.empty(blocks * d + 2 * blocks + 4, device=device, dtype=torch.float32)
-        self.counter = torch.zeros(1, device=device, dtype=torch.int32)
         self.loss = torch.zeros(1, device=device, dtype=torch.float64)
 
     def __call__(self, X, y, theta, g, logistic: bool = True):
@@ -21,7 +20,7 @@ class DenseGrad:
         n, d = X.shape
         assert d == self.d and g.numel() >= d
         _lib.call("pcl_lr_dense_grad", X, y, theta, n, d, int(logistic), g, self.loss, self.scratch,
-                  self.counter, self.blocks, _lib.stream_ptr())
+                  self.blocks, _lib.stream_ptr())
         return self.loss
 
 

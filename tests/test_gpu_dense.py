@@ -232,3 +232,24 @@ def test_pagerank_gpu_matches_power_iteration():
     pr.step(track_delta=True)
     assert float(pr.delta_l1.item()) >= 0.0
     pr.free()
+
+
+@pytest.mark.parametrize("d", [1, 4, 31, 127, 128, 130, 256, 257, 512, 513, 1024, 1025, 6000])
+def test_dense_gradient_at_the_edges_of_its_row_kernels(d):
+    """Row lengths around the register forms (aligned and not), row counts around a warp's step."""
+    from paracel_b200.ops.linear import DenseGrad
+    g = torch.Generator(device="cuda").manual_seed(d)
+    op = DenseGrad(d, "cuda")
+    for n in (1, 3, 8, 33, 2001):
+        for lead in (0, 1):                       # lead 1: rows off their 16-byte boundaries
+            X = torch.randn(n * d + lead, device="cuda", generator=g)[lead:].view(n, d)
+            theta = torch.randn(d, device="cuda", generator=g) / d ** 0.5
+            y = torch.randn(n, device="cuda", generator=g)
+            grad = torch.empty(d, device="cuda")
+            loss = op(X, y, theta, grad, logistic=False)
+            X64, r = X.double(), y.double() - X.double() @ theta.double()
+            # a residual is off by d + 1 roundings of its terms, a sum of n products by n + 2 more
+            dr = (d + 2) * 2.0 ** -24 * (X64.abs() @ theta.double().abs() + y.double().abs())
+            bound = X64.abs().T @ dr + (n + 2) * 2.0 ** -24 * (X64.abs().T @ r.abs())
+            assert bool(((grad.double() - X64.T @ r).abs() <= bound).all()), (n, lead)
+            assert abs(float(loss) - float((r * r).sum())) <= float((2 * r.abs() * dr + dr * dr).sum()) + 1e-12
