@@ -14,7 +14,7 @@
 //                      slot, and the last one to arrive solves
 // The dual form needs lambda > 0 (with lambda <= 0 every user takes the last form).
 // Rank 128, 100 k users, 10 M Zipf(1.1) ratings: 84 % of the users have at most 32 ratings and
-// 4.6 % more than 128, while those hold 82 % of the ratings; a solve takes 6.9 ms against 36.1 ms
+// 4.6 % more than 128, while those hold 82 % of the ratings; a solve takes 6.5 ms against 36.1 ms
 // with the k x k form for everyone, of which two thirds were its 128 x 128 factorisations.
 #include <cuda_pipeline.h>
 
@@ -22,8 +22,8 @@
 
 namespace {
 
-constexpr int NT = 320;            // threads of a CTA: ten warps (ten 32 x 32 blocks of a 128 x 128 triangle)
-constexpr int RS = 20;             // item rows per stage of the Gram loop, two per warp
+constexpr int NT = 192;            // threads of a CTA: six warps (six 32 x 64 blocks cover a 128 x 128 triangle)
+constexpr int RS = 24;             // item rows per stage of the Gram loop, four per warp
 
 // lists and counters the plan kernel writes
 enum { C_BIG = 0, C_SMALL = 1, C_SLOT = 2, C_T16 = 3, C_T32 = 4, C_T64 = 5, C_T96 = 6, C_TICKET = 7, C_N = 8 };
@@ -49,6 +49,23 @@ struct AlsArgs {
   float lambda;
   int vec;                         // rows of H start on 16-byte boundaries and k is a multiple of 4
 };
+
+// Two fp32 multiply-adds in one instruction.  The fp32 pipe takes as long for one as for two: the Gram
+// loop below took 5.9 ms with scalar multiply-adds and 4.9 ms with these (rank 128, 8.5 M ratings).
+typedef unsigned long long u64;
+__device__ __forceinline__ u64 pack2(float x, float y) {
+  u64 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void unpack2(u64 v, float& x, float& y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+  u64 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
 
 // ------------------------------------------------------------------------------------------ plan
 __global__ void __launch_bounds__(256) als_plan_kernel(AlsArgs a) {
@@ -129,14 +146,14 @@ __device__ __forceinline__ void diag_factor(float* sA, int LD, float* s_inv, int
 //
 // Blocked right-looking Cholesky in panels of 16 columns with two barriers a panel.  The
 // right-hand side travels as one more row, so the forward substitution comes with the
-// factorisation; warp 9 updates and factors the next diagonal block while warps 0 to 7 update the
-// rest of the trailing matrix and warp 8 the right-hand side.  What bounds it is that chain of
+// factorisation; warp 5 updates and factors the next diagonal block while warps 0 to 3 update the
+// rest of the trailing matrix and warp 4 the right-hand side.  What bounds it is that chain of
 // dependent steps, hidden by the other CTAs of the SM.
 template <int MB>
 __device__ __forceinline__ void chol_solve(float* sA, int LD, float* s_inv, int panels, int tid) {
   const int lane = tid & 31, warp = tid >> 5;
   const int Kd = 16 * panels;
-  if (warp == 9) diag_factor(sA, LD, s_inv, 0, lane);
+  if (warp == 5) diag_factor(sA, LD, s_inv, 0, lane);
   __syncthreads();
   for (int j0 = 0; j0 < Kd; j0 += 16) {
     const int j1 = j0 + 16, m = Kd - j1;
@@ -155,35 +172,39 @@ __device__ __forceinline__ void chol_solve(float* sA, int LD, float* s_inv, int 
     }
     __syncthreads();
     if (m == 0) break;
-    if (warp < 8) {                        // A22 -= L21 L21^T below the diagonal, all but block (0, 0)
+    if (warp < 4) {                        // A22 -= L21 L21^T below the diagonal, all but block (0, 0)
+      // rows ty + 8 i, columns tx + 16 j: j <= i / 2
       constexpr int TB = MB > 1 ? MB - 1 : 1;
       const int tx = tid & 15, ty = tid >> 4, mb = m >> 4;
-      float t[TB * (TB + 1) / 2];
+      float t[TB * (TB + 1)];
 #pragma unroll
-      for (int e = 0; e < TB * (TB + 1) / 2; ++e) t[e] = 0.f;
-#pragma unroll 4
+      for (int e = 0; e < TB * (TB + 1); ++e) t[e] = 0.f;
+#pragma unroll 2
       for (int q = 0; q < 16; ++q) {
-        float lr[TB], lc[TB];
+        float lc[TB];
 #pragma unroll
-        for (int i = 0; i < TB; ++i) {
-          lr[i] = i < mb ? sA[(j1 + ty + 16 * i) * LD + j0 + q] : 0.f;
-          lc[i] = i < mb ? sA[(j1 + tx + 16 * i) * LD + j0 + q] : 0.f;
-        }
+        for (int i = 0; i < TB; ++i) lc[i] = i < mb ? sA[(j1 + tx + 16 * i) * LD + j0 + q] : 0.f;
 #pragma unroll
         for (int i = 1; i < TB; ++i)
           if (i < mb) {
 #pragma unroll
-            for (int j = 0; j <= i; ++j) t[i * (i + 1) / 2 + j] = fmaf(lr[i], lc[j], t[i * (i + 1) / 2 + j]);
+            for (int h = 0; h < 2; ++h) {
+              const float lr = sA[(j1 + ty + 16 * i + 8 * h) * LD + j0 + q];
+#pragma unroll
+              for (int j = 0; j <= i; ++j) t[i * (i + 1) + 2 * j + h] = fmaf(lr, lc[j], t[i * (i + 1) + 2 * j + h]);
+            }
           }
       }
 #pragma unroll
       for (int i = 1; i < TB; ++i)
 #pragma unroll
-        for (int j = 0; j <= i; ++j) {
-          const int r = j1 + ty + 16 * i, c = j1 + tx + 16 * j;
-          if (i < mb && c <= r) sA[r * LD + c] -= t[i * (i + 1) / 2 + j];
-        }
-    } else if (warp == 8) {
+        for (int j = 0; j <= i; ++j)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int r = j1 + ty + 16 * i + 8 * h, c = j1 + tx + 16 * j;
+            if (i < mb && c <= r) sA[r * LD + c] -= t[i * (i + 1) + 2 * j + h];
+          }
+    } else if (warp == 4) {
       for (int c = lane; c < m; c += 32) {
         float v = sA[Kd * LD + j1 + c];
 #pragma unroll
@@ -237,42 +258,27 @@ __device__ __forceinline__ void chol_solve(float* sA, int LD, float* s_inv, int 
 }
 
 // ---------------------------------------------------------------------------------- primal form
-typedef unsigned long long u64;
-__device__ __forceinline__ u64 pack2(float x, float y) {
-  u64 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-  return r;
-}
-__device__ __forceinline__ void unpack2(u64 v, float& x, float& y) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
-}
-__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
-  u64 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-
-// The Gram matrix is bound by fp32 arithmetic: 32 x 32 blocks of its lower triangle, one per warp
-// (10 of 16 blocks at K = 128; with fewer blocks several warps share one and split the rows), 4 x 8
-// values per lane as packed pairs, fed by three conflict-free 16-byte shared-memory loads per item
-// row.  Item rows arrive by asynchronous copies two stages ahead.
-template <int KB>
+// 32 x 64 blocks of the lower triangle (32 x 32 at K = 32), one per warp; with fewer than six blocks
+// several warps share one and split the rows.  A lane owns 8 x 8 values, so an item row costs it four
+// 16-byte shared-memory loads for 64 multiply-adds.  A 16-byte load takes four passes of the shared
+// memory however many lanes read the same word, and with 4 x 8 values per lane (ten 32 x 32 blocks)
+// those passes were the bound: 77 % of all cycles, 174 cycles a rating against 167 here.
+// Item rows arrive by asynchronous copies two stages ahead.
+template <int K>
 __global__ void __launch_bounds__(NT, 3) als_primal_kernel(AlsArgs a) {
-  constexpr int K = 16 * KB, LD = K + 1, B = KB / 2, NB = B * (B + 1) / 2, GR = 10 / NB;
+  constexpr int LD = K + 1;
+  constexpr int CW = K == 32 ? 1 : 2;                      // 16-byte pieces of columns per lane
+  constexpr int NB = K == 32 ? 1 : (K == 64 ? 2 : 6), GR = 6 / NB;
   extern __shared__ __align__(16) float sm[];
   float* sA = sm;                       // (K + 1) x LD, under it three stages of RS x K item rows
   __shared__ float s_inv[K];
   __shared__ float s_r[3][RS];
-  __shared__ float s_b[2][K];
   __shared__ int s_seg;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int panels = (a.k + 15) / 16, Kd = 16 * panels;
-  const int blk = warp % NB, grp = warp / NB;      // warps from NB * GR on have no block
-  const bool has_blk = grp < GR;
-  int bi = 0;
-  while ((bi + 1) * (bi + 2) / 2 <= blk) ++bi;
-  const int bj = blk - bi * (bi + 1) / 2;
-  const int row0 = 32 * bi + 4 * (lane >> 2), col0 = 32 * bj + 4 * (lane & 3);
+  const int blk = warp % NB, grp = warp / NB;
+  const int bi = blk < 4 ? blk : blk - 2, bj = blk < 4 ? 0 : 1;   // (0..3, 0), (2..3, 1)
+  const int row0 = 32 * bi + 8 * (lane >> 3), col0 = 64 * bj + 4 * (lane & 7);
   const int n_big = a.counters[C_BIG], n_seg = n_big + a.counters[C_SMALL];
   for (;;) {
     __syncthreads();                    // the previous system is done with shared memory
@@ -288,25 +294,25 @@ __global__ void __launch_bounds__(NT, 3) als_primal_kernel(AlsArgs a) {
     const int ns = (cnt + RS - 1) / RS;
     if (a.k < K)                        // columns behind the rank stay zero in every stage
       for (int e = tid; e < 3 * RS * (K - a.k); e += NT) sm[(e / (K - a.k)) * K + a.k + e % (K - a.k)] = 0.f;
-    u64 acc[4][4];
+    u64 acc[8][2 * CW];                 // pairs of neighbouring columns
+    float b1 = 0.f;                     // entry tid of H^T a
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
-    float bacc = 0.f;                   // entry tid % K of H^T a over half of the rows
-    int idx[2];                         // item rows of the warp's two rows of the stage to come
+      for (int j = 0; j < 2 * CW; ++j) acc[i][j] = 0ull;
+    int idx[4];                         // item rows of the warp's rows of the stage to come
     auto fetch_idx = [&](int s) {
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int r = s * RS + warp + 10 * q;
+      for (int q = 0; q < 4; ++q) {
+        const int r = s * RS + warp + 6 * q;
         idx[q] = r < cnt ? __ldg(a.item_idx + p0 + r) : -1;
       }
     };
     auto stage = [&](int s) {
       if (s < ns) {
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const int r = warp + 10 * q;
+        for (int q = 0; q < 4; ++q) {
+          const int r = warp + 6 * q;
           stage_row(sm + ((s % 3) * RS + r) * K, idx[q] >= 0 ? a.H + (long long)idx[q] * a.k : nullptr, a.H, a.k,
                     a.vec, lane);
           if (lane == 0)
@@ -327,44 +333,44 @@ __global__ void __launch_bounds__(NT, 3) als_primal_kernel(AlsArgs a) {
       stage(s + 2);
       fetch_idx(s + 3);
       const float* sh = sm + (s % 3) * RS * K;
-      if (has_blk) {
 #pragma unroll 2
-        for (int r = grp; r < RS; r += GR) {
-          const float4 h = *reinterpret_cast<const float4*>(sh + r * K + row0);
-          const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(sh + r * K + col0);
-          const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(sh + r * K + col0 + 16);
-          const u64 hh[4] = {pack2(h.x, h.x), pack2(h.y, h.y), pack2(h.z, h.z), pack2(h.w, h.w)};
+      for (int r = grp; r < RS; r += GR) {
+        const float4 h0 = *reinterpret_cast<const float4*>(sh + r * K + row0);
+        const float4 h1 = *reinterpret_cast<const float4*>(sh + r * K + row0 + 4);
+        u64 x[2 * CW];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            acc[i][0] = fma2(hh[i], x.x, acc[i][0]);
-            acc[i][1] = fma2(hh[i], x.y, acc[i][1]);
-            acc[i][2] = fma2(hh[i], y.x, acc[i][2]);
-            acc[i][3] = fma2(hh[i], y.y, acc[i][3]);
-          }
+        for (int w = 0; w < CW; ++w) {
+          const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(sh + r * K + col0 + 32 * w);
+          x[2 * w] = v.x; x[2 * w + 1] = v.y;
+        }
+        const float h[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const u64 hh = pack2(h[i], h[i]);
+#pragma unroll
+          for (int j = 0; j < 2 * CW; ++j) acc[i][j] = fma2(hh, x[j], acc[i][j]);
         }
       }
-      if (tid < 2 * K) {
-        const int c = tid % K, r0 = tid / K * (RS / 2);
-#pragma unroll
-        for (int r = 0; r < RS / 2; ++r) bacc = fmaf(s_r[s % 3][r0 + r], sh[(r0 + r) * K + c], bacc);
+      if (tid < K) {
+#pragma unroll 8
+        for (int r = 0; r < RS; ++r) b1 = fmaf(s_r[s % 3][r], sh[r * K + tid], b1);
       }
     }
     __pipeline_wait_prior(0);
     bool mine = true;                   // this warp's sums go into the matrix
     if (slot >= 0) {
       float* gA = a.scratch + (long long)slot * (K * K + K);
-      if (has_blk) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+      for (int w = 0; w < CW; ++w) {
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            float4 v;
-            unpack2(acc[i][2 * h], v.x, v.y);
-            unpack2(acc[i][2 * h + 1], v.z, v.w);
-            pcl_red_add4(gA + (row0 + i) * K + col0 + 16 * h, v);
-          }
+        for (int i = 0; i < 8; ++i) {
+          float4 v;
+          unpack2(acc[i][2 * w], v.x, v.y);
+          unpack2(acc[i][2 * w + 1], v.z, v.w);
+          pcl_red_add4(gA + (row0 + i) * K + col0 + 32 * w, v);
+        }
       }
-      if (tid < 2 * K) atomicAdd(gA + K * K + tid % K, bacc);
+      if (tid < K) atomicAdd(gA + K * K + tid, b1);
       __threadfence();
       __syncthreads();
       if (tid == 0) {
@@ -377,48 +383,50 @@ __global__ void __launch_bounds__(NT, 3) als_primal_kernel(AlsArgs a) {
       mine = grp == 0;
       if (mine) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int w = 0; w < CW; ++w) {
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const float4 v = __ldcg(reinterpret_cast<const float4*>(gA + (row0 + i) * K + col0 + 16 * h));
-            acc[i][2 * h] = pack2(v.x, v.y);
-            acc[i][2 * h + 1] = pack2(v.z, v.w);
+          for (int i = 0; i < 8; ++i) {
+            const float4 v = __ldcg(reinterpret_cast<const float4*>(gA + (row0 + i) * K + col0 + 32 * w));
+            acc[i][2 * w] = pack2(v.x, v.y);
+            acc[i][2 * w + 1] = pack2(v.z, v.w);
           }
+        }
       }
-      if (tid < 2 * K) bacc = tid < K ? __ldcg(gA + K * K + tid) : 0.f;
+      if (tid < K) b1 = __ldcg(gA + K * K + tid);
     }
     __syncthreads();                    // everyone is done with the last stage
-    if (tid < 2 * K) s_b[tid / K][tid % K] = bacc;
 #pragma unroll 1
     for (int g = 0; g < GR; ++g) {      // warps that share a block add one after the other
-      if (has_blk && grp == g && mine) {
+      if (grp == g && mine) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float v[2];
-            unpack2(acc[i][j], v[0], v[1]);
+          for (int w = 0; w < CW; ++w) {
+            float v[4];
+            unpack2(acc[i][2 * w], v[0], v[1]);
+            unpack2(acc[i][2 * w + 1], v[2], v[3]);
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              const int r = row0 + i, c = col0 + 16 * (j >> 1) + 2 * (j & 1) + q;
-              if (g == 0) sA[r * LD + c] = v[q] + (r == c ? a.lambda : 0.f);
-              else sA[r * LD + c] += v[q];
+            for (int j = 0; j < 4; ++j) {
+              const int r = row0 + i, c = col0 + 32 * w + j;
+              if (c > r) continue;      // a block reaches past the diagonal: its other half is not needed
+              if (g == 0) sA[r * LD + c] = v[j] + (r == c ? a.lambda : 0.f);
+              else sA[r * LD + c] += v[j];
             }
           }
       }
       __syncthreads();
     }
-    if (tid < Kd) sA[Kd * LD + tid] = s_b[0][tid] + s_b[1][tid];
+    if (tid < Kd) sA[Kd * LD + tid] = b1;
     __syncthreads();
-    chol_solve<KB>(sA, LD, s_inv, panels, tid);
+    chol_solve<K / 16>(sA, LD, s_inv, panels, tid);
     if (tid < a.k) a.W[(long long)u * a.k + tid] = sA[Kd * LD + tid];
   }
 }
 
 // --------------------------------------------------------------------- dual form, CTA per user
 template <int NB2>                      // n <= 32 * NB2
-__global__ void __launch_bounds__(NT, 2) als_dual_kernel(AlsArgs a, int cls) {
-  constexpr int N = 32 * NB2, LD = N + 1, NB = NB2 * (NB2 + 1) / 2, GR = 10 / NB;
+__global__ void __launch_bounds__(NT, 3) als_dual_kernel(AlsArgs a, int cls) {
+  constexpr int N = 32 * NB2, LD = N + 1, NB = NB2 * (NB2 + 1) / 2, GR = 6 / NB;   // three or six 32 x 32 blocks
   extern __shared__ __align__(16) float sm[];
   const int KS = (a.k + 31) / 32 * 32 + 4;         // row pitch: eight rows four banks apart
   float* sh = sm;                       // N x KS item rows
@@ -426,7 +434,6 @@ __global__ void __launch_bounds__(NT, 2) als_dual_kernel(AlsArgs a, int cls) {
   __shared__ float s_inv[N];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int blk = warp % NB, grp = warp / NB;
-  const bool has_blk = grp < GR;
   int bi = 0;
   while ((bi + 1) * (bi + 2) / 2 <= blk) ++bi;
   const int bj = blk - bi * (bi + 1) / 2;
@@ -446,32 +453,36 @@ __global__ void __launch_bounds__(NT, 2) als_dual_kernel(AlsArgs a, int cls) {
     __pipeline_wait_prior(0);
     __syncthreads();
     float acc[4][8];
+    {
+      u64 acc2[4][8];                   // sums over even and odd components
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-    if (has_blk) {
+        for (int j = 0; j < 8; ++j) acc2[i][j] = 0ull;
 #pragma unroll 1
       for (int c = grp; c < k4; c += GR) {
-        float4 x[4];
+        ulonglong2 x[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(sh + (row0 + 8 * i) * KS + 4 * c);
+        for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const ulonglong2*>(sh + (row0 + 8 * i) * KS + 4 * c);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const float4 y = *reinterpret_cast<const float4*>(sh + (col0 + 4 * j) * KS + 4 * c);
+          const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(sh + (col0 + 4 * j) * KS + 4 * c);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            acc[i][j] = fmaf(x[i].x, y.x, acc[i][j]);
-            acc[i][j] = fmaf(x[i].y, y.y, acc[i][j]);
-            acc[i][j] = fmaf(x[i].z, y.z, acc[i][j]);
-            acc[i][j] = fmaf(x[i].w, y.w, acc[i][j]);
-          }
+          for (int i = 0; i < 4; ++i) acc2[i][j] = fma2(x[i].y, y.y, fma2(x[i].x, y.x, acc2[i][j]));
         }
       }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float e, o;
+          unpack2(acc2[i][j], e, o);
+          acc[i][j] = e + o;
+        }
     }
 #pragma unroll 1
     for (int g = 0; g < GR; ++g) {
-      if (has_blk && grp == g) {
+      if (grp == g) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -528,27 +539,22 @@ __global__ void __launch_bounds__(128) als_warp_kernel(AlsArgs a, int cls) {
     __pipeline_commit();
     __pipeline_wait_prior(0);
     __syncwarp();
-    float acc[RI][CJ];
+    u64 acc[RI][CJ];                    // sums over even and odd components
 #pragma unroll
     for (int i = 0; i < RI; ++i)
 #pragma unroll
-      for (int j = 0; j < CJ; ++j) acc[i][j] = 0.f;
+      for (int j = 0; j < CJ; ++j) acc[i][j] = 0ull;
     const int r0 = lane >> 2, c0 = lane & 3;
 #pragma unroll 1
     for (int c = 0; c < k4; ++c) {
-      float4 x[RI];
+      ulonglong2 x[RI];
 #pragma unroll
-      for (int i = 0; i < RI; ++i) x[i] = *reinterpret_cast<const float4*>(sh + (r0 + 8 * i) * KS + 4 * c);
+      for (int i = 0; i < RI; ++i) x[i] = *reinterpret_cast<const ulonglong2*>(sh + (r0 + 8 * i) * KS + 4 * c);
 #pragma unroll
       for (int j = 0; j < CJ; ++j) {
-        const float4 y = *reinterpret_cast<const float4*>(sh + (c0 + 4 * j) * KS + 4 * c);
+        const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(sh + (c0 + 4 * j) * KS + 4 * c);
 #pragma unroll
-        for (int i = 0; i < RI; ++i) {
-          acc[i][j] = fmaf(x[i].x, y.x, acc[i][j]);
-          acc[i][j] = fmaf(x[i].y, y.y, acc[i][j]);
-          acc[i][j] = fmaf(x[i].z, y.z, acc[i][j]);
-          acc[i][j] = fmaf(x[i].w, y.w, acc[i][j]);
-        }
+        for (int i = 0; i < RI; ++i) acc[i][j] = fma2(x[i].y, y.y, fma2(x[i].x, y.x, acc[i][j]));
       }
     }
 #pragma unroll
@@ -556,7 +562,9 @@ __global__ void __launch_bounds__(128) als_warp_kernel(AlsArgs a, int cls) {
 #pragma unroll
       for (int j = 0; j < CJ; ++j) {
         const int r = r0 + 8 * i, c = c0 + 4 * j;
-        sG[r * LG + c] = acc[i][j] + (r == c ? a.lambda : 0.f);
+        float e, o;
+        unpack2(acc[i][j], e, o);
+        sG[r * LG + c] = e + o + (r == c ? a.lambda : 0.f);
       }
     __syncwarp();
     float g[N];
@@ -631,16 +639,15 @@ int resident_grid(F kernel, int threads, size_t smem, long long need, int* grid)
   return 0;
 }
 
-template <int KB>
+template <int K>
 int launch_primal(const AlsArgs& a, long long max_seg, cudaStream_t stream) {
-  constexpr int K = 16 * KB;
   size_t smem = (size_t)(K + 1) * (K + 1) * sizeof(float);
   if (smem < (size_t)3 * RS * K * sizeof(float)) smem = (size_t)3 * RS * K * sizeof(float);
   int grid = 0;
-  const int rc = resident_grid(als_primal_kernel<KB>, NT, smem, max_seg, &grid);
+  const int rc = resident_grid(als_primal_kernel<K>, NT, smem, max_seg, &grid);
   if (rc != 0) return rc;
   als_clear_kernel<<<148 * 4, 256, 0, stream>>>(a.scratch, a.counters, K * K + K);
-  als_primal_kernel<KB><<<grid, NT, smem, stream>>>(a);
+  als_primal_kernel<K><<<grid, NT, smem, stream>>>(a);
   return pcl_last_error();
 }
 
@@ -671,7 +678,7 @@ int launch_warp(const AlsArgs& a, int cls, cudaStream_t stream) {
 
 // k <= 128, n_users < 2^31.  `nnz` is the length of item_idx / rating (user_ptr is ascending within
 // [0, nnz]).  Users with more than `split` ratings are cut into pieces of `piece`.  Workspaces:
-// scratch holds nnz / split slots of K*K + K floats (K = k rounded up to 32 / 64 / 96 / 128, 16-byte
+// scratch holds nnz / split slots of K*K + K floats (K = k rounded up to 32 / 64 / 128, 16-byte
 // aligned) and slot_count as many ints; counters 8 ints; seg 3 x seg_cap ints with
 // seg_cap >= n_users + nnz / piece + nnz / split; user_list 4 x n_users ints.  Rows of W of users without
 // ratings are not written.
@@ -689,10 +696,9 @@ PCL_API int pcl_als_solve(const long long* user_ptr, const int* item_idx, const 
   als_plan_kernel<<<(int)((n_users + 255) / 256), 256, 0, stream>>>(a);
   int rc = pcl_last_error();
   if (rc != 0) return rc;
-  if (k <= 32) rc = launch_primal<2>(a, seg_cap, stream);
-  else if (k <= 64) rc = launch_primal<4>(a, seg_cap, stream);
-  else if (k <= 96) rc = launch_primal<6>(a, seg_cap, stream);
-  else rc = launch_primal<8>(a, seg_cap, stream);
+  if (k <= 32) rc = launch_primal<32>(a, seg_cap, stream);
+  else if (k <= 64) rc = launch_primal<64>(a, seg_cap, stream);
+  else rc = launch_primal<128>(a, seg_cap, stream);
   if (rc != 0 || !(lambda > 0.f)) return rc;
   if (k > 64 && (rc = launch_dual<3>(a, 3, stream)) != 0) return rc;
   if (k > 33 && (rc = launch_dual<2>(a, 2, stream)) != 0) return rc;

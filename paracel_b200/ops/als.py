@@ -7,7 +7,7 @@ from . import _lib
 
 
 def _kpad(k: int) -> int:
-    for K in (32, 64, 96, 128):
+    for K in (32, 64, 128):
         if k <= K:
             return K
     raise ValueError("factor rank above 128 is not supported")
