@@ -269,11 +269,21 @@ int launch_rows_times(const float* M, long long n, int K, const float* P, float*
 // out[i] = scale * u_i + shift with u_i = (word_i mod 2^24) / 2^24 for the words of the Mersenne Twister
 // MT19937 (Matsumoto and Nishimura, 1998) after init_genrand(seed): the stream of the host
 // generator, made where it is used.
-// One block: 227 words of the recurrence are independent of one another, so a step makes 227 and ends
-// with a barrier; tempering and the store are off that chain.
-__global__ void __launch_bounds__(256) mt19937_kernel(float* __restrict__ out, long long n, unsigned seed,
-                                                      float scale, float shift) {
-  __shared__ unsigned x[1024];           // word k at k mod 1024: the last 624 and the 227 in the making
+// One block and one chain of steps.  x[k + 624] = x[k + 397] ^ f(x[k], x[k + 1]) gives 227 words a step;
+// putting the recurrence in for x[k + 397] and again for x[k + 170],
+//   x[k + 624] = x[k - 57] ^ f(x[k - 454], x[k - 453]) ^ f(x[k - 227], x[k - 226]) ^ f(x[k], x[k + 1]),
+// gives 623, and the barrier that ends a step is what a step costs.  The words of a step are tempered
+// and stored under the loads of the next.  3.2 M numbers: 1.54 ms with 227 words a step.
+constexpr int MT_T = 640, MT_W = 623;
+
+__device__ __forceinline__ unsigned mt_f(unsigned a, unsigned b) {
+  const unsigned y = (a & 0x80000000u) | (b & 0x7fffffffu);
+  return (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
+}
+
+__global__ void __launch_bounds__(MT_T) mt19937_kernel(float* __restrict__ out, long long n, unsigned seed,
+                                                       float scale, float shift) {
+  __shared__ unsigned x[2048];           // word k at k mod 2048: a step reads 1078 back and writes 623
   const int t = threadIdx.x;
   if (t == 0) {
     unsigned s = seed;
@@ -284,76 +294,105 @@ __global__ void __launch_bounds__(256) mt19937_kernel(float* __restrict__ out, l
     }
   }
   __syncthreads();
-  for (long long i0 = 0; i0 < n; i0 += 227) {
+  auto emit = [&](long long i, unsigned v) {
+    v ^= v >> 11;
+    v ^= (v << 7) & 0x9d2c5680u;
+    v ^= (v << 15) & 0xefc60000u;
+    v ^= v >> 18;
+    if (i < n) out[i] = fmaf((float)(v & 0xffffffu) * (1.f / 16777216.f), scale, shift);
+  };
+  // words 624 .. 1077 by the recurrence itself: the long form reads 454 words before the state
+  for (int k0 = 0; k0 < 454; k0 += 227) {
     if (t < 227) {
-      const int k = (int)((i0 + t) & 1023);
-      const unsigned y = (x[k] & 0x80000000u) | (x[(k + 1) & 1023] & 0x7fffffffu);
-      unsigned v = x[(k + 397) & 1023] ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
-      x[(k + 624) & 1023] = v;
-      v ^= v >> 11;
-      v ^= (v << 7) & 0x9d2c5680u;
-      v ^= (v << 15) & 0xefc60000u;
-      v ^= v >> 18;
-      if (i0 + t < n) out[i0 + t] = fmaf((float)(v & 0xffffffu) * (1.f / 16777216.f), scale, shift);
+      const unsigned v = x[k0 + t + 397] ^ mt_f(x[k0 + t], x[k0 + t + 1]);
+      x[k0 + t + 624] = v;
+      emit(k0 + t, v);
+    }
+    __syncthreads();
+  }
+  unsigned last = 0;
+  for (long long i0 = 454; i0 < n + MT_W; i0 += MT_W) {   // the last step only stores
+    if (t < MT_W) {
+      const int k = (int)((i0 + t) & 2047);
+      auto w = [&](int d) { return x[(k + d) & 2047]; };
+      const unsigned a0 = w(-454), a1 = w(-453), b0 = w(-227), b1 = w(-226), c0 = w(0), c1 = w(1), e = w(-57);
+      if (i0 > 454) emit(i0 - MT_W + t, last);
+      last = e ^ mt_f(a0, a1) ^ mt_f(b0, b1) ^ mt_f(c0, c1);
+      x[(k + 624) & 2047] = last;
     }
     __syncthreads();
   }
 }
 
-// One CTA.  Shared memory: L (K x K doubles) and X = L^-1 (K x K doubles).
-__global__ void __launch_bounds__(256) chol_factor_kernel(const float* __restrict__ G, int K,
-                                                          float* __restrict__ T, float* __restrict__ R,
-                                                          double rel_tol, int* __restrict__ info) {
+// One CTA of CH_T threads.  Shared memory: L (K x K doubles) and X = L^-1 (K x K doubles).  Everything is a
+// chain over the columns: two barriers a column in the factorisation, and a warp per column of the
+// inverse that eliminates as it goes (with one thread per column and dot products, the first
+// column's chain of K^2 / 2 dependent multiply-adds was most of 40 us at K = 32; 30 us now).
+constexpr int CH_T = 512;
+
+__global__ void __launch_bounds__(CH_T) chol_factor_kernel(const float* __restrict__ G, int K,
+                                                           float* __restrict__ T, float* __restrict__ R,
+                                                           double rel_tol, int* __restrict__ info) {
   extern __shared__ double sd[];
   double* L = sd;
   double* X = sd + (size_t)K * K;
-  __shared__ double s_diag, s_max;
-  __shared__ int s_bad;
-  const int tid = threadIdx.x, nt = blockDim.x;
+  __shared__ double s_col[112], s_inv[112], s_max;
+  const int tid = threadIdx.x, nt = CH_T, lane = tid & 31, warp = tid >> 5;
   for (int e = tid; e < K * K; e += nt) {
     const int i = e / K, j = e % K;
     L[e] = 0.5 * ((double)G[i * K + j] + (double)G[j * K + i]);   // symmetrise
-    X[e] = 0.0;
   }
-  if (tid == 0) { s_bad = 0; s_max = 0.0; }
   __syncthreads();
-  if (tid == 0) {
+  if (warp == 0) {
     double m = 0.0;
-    for (int i = 0; i < K; ++i) m = fmax(m, fabs(L[i * K + i]));
-    s_max = m;
+    for (int i = lane; i < K; i += 32) m = fmax(m, fabs(L[i * K + i]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0) s_max = m;
   }
   __syncthreads();
   // right-looking Cholesky on the lower triangle
+  const double tol = rel_tol * s_max;
+  const int tx = tid & 15, ty = tid >> 4;       // 16 columns x 32 rows of the trailing matrix
   for (int j = 0; j < K; ++j) {
-    if (tid == 0) {
-      const double d = L[j * K + j];
-      if (!(d > rel_tol * s_max) && s_bad == 0) s_bad = j + 1;
-      s_diag = d > 0.0 ? sqrt(d) : 1.0;
+    const double d = L[j * K + j];
+    if (!(d > tol)) {                           // the same for every thread
+      if (tid == 0) *info = j + 1;
+      return;
     }
+    // column j of the factor goes to a buffer of its own: its place is read by the threads still here
+    const double inv = 1.0 / sqrt(d);
+    if (tid == 0) s_inv[j] = inv;
+    for (int i = j + tid; i < K; i += nt) s_col[i] = i == j ? d * inv : L[i * K + j] * inv;
     __syncthreads();
-    if (s_bad) break;
-    const double dj = s_diag;
-    for (int i = j + tid; i < K; i += nt) L[i * K + j] = (i == j) ? dj : L[i * K + j] / dj;
-    __syncthreads();
-    // trailing update: L[i][k] -= L[i][j] * L[k][j] for j < k <= i
-    const int rem = K - j - 1;
-    for (int e = tid; e < rem * rem; e += nt) {
-      const int i = j + 1 + e / rem, k = j + 1 + e % rem;
-      if (k <= i) L[i * K + k] -= L[i * K + j] * L[k * K + j];
-    }
+    for (int i = j + tid; i < K; i += nt) L[i * K + j] = s_col[i];
+    for (int i = j + 1 + ty; i < K; i += CH_T / 16)
+      for (int k = j + 1 + tx; k <= i; k += 16) L[i * K + k] -= s_col[i] * s_col[k];
     __syncthreads();
   }
-  if (s_bad) {
-    if (tid == 0) *info = s_bad;
-    return;
-  }
-  // X = L^-1 by forward substitution, one column per thread
-  for (int c = tid; c < K; c += nt) {
-    for (int i = c; i < K; ++i) {
-      double s = (i == c) ? 1.0 : 0.0;
-      for (int k = c; k < i; ++k) s -= L[i * K + k] * X[k * K + c];
-      X[i * K + c] = s / L[i * K + i];
+  // X = L^-1, a warp per column: lane l holds rows l, l + 32, ... of the column
+  for (int c = warp; c < K; c += nt / 32) {
+    double b[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) b[q] = lane + 32 * q == c ? 1.0 : 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      for (int l = 0; l < 32; ++l) {
+        const int k = 32 * q + l;
+        if (k >= K) break;
+        if (k < c) continue;
+        const double x = __shfl_sync(0xffffffffu, b[q], l) * s_inv[k];
+        if (lane == l) b[q] = x;
+#pragma unroll
+        for (int p = q; p < 4; ++p) {
+          const int i = lane + 32 * p;
+          if (i > k && i < K) b[p] -= L[i * K + k] * x;
+        }
+      }
     }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (lane + 32 * q < K) X[(lane + 32 * q) * K + c] = lane + 32 * q >= c ? b[q] : 0.0;
   }
   __syncthreads();
   for (int e = tid; e < K * K; e += nt) {
@@ -404,7 +443,7 @@ PCL_API int pcl_rows_times(const float* M, long long n, int K, const float* P, i
 PCL_API int pcl_mt19937_uniform(float* out, long long n, unsigned int seed, float scale, float shift,
                                 cudaStream_t stream) {
   if (n <= 0) return 0;
-  mt19937_kernel<<<1, 256, 0, stream>>>(out, n, seed, scale, shift);
+  mt19937_kernel<<<1, MT_T, 0, stream>>>(out, n, seed, scale, shift);
   return pcl_last_error();
 }
 
@@ -415,6 +454,6 @@ PCL_API int pcl_chol_factor(const float* G, int K, float* T, float* R, double re
   cudaError_t e = cudaFuncSetAttribute(chol_factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
   if (e != cudaSuccess) return (int)e;
-  chol_factor_kernel<<<1, 256, smem, stream>>>(G, K, T, R, rel_tol, info);
+  chol_factor_kernel<<<1, CH_T, smem, stream>>>(G, K, T, R, rel_tol, info);
   return pcl_last_error();
 }

@@ -342,7 +342,7 @@ def test_rows_times_matches_fp64(K):
         assert bool(((two.double() - M.double() @ P64 @ P64.T).abs() <= bound).all())
 
 
-@pytest.mark.parametrize("n,seed", [(1, 0), (226, 3), (227, 3), (228, 7), (1023, 2 ** 32 - 1), (100_003, -5)])
+@pytest.mark.parametrize("n,seed", [(1, 0), (226, 3), (227, 3), (228, 7), (454, 1), (455, 2), (1077, 3), (1078, 4), (1023, 2 ** 32 - 1), (100_003, -5)])
 def test_host_rand_is_the_cpu_generators_stream(n, seed):
     from paracel_b200.ops.svd import host_rand
     g = torch.Generator()
