@@ -25,6 +25,15 @@ struct PrArgs {
   int n_heavy;
 };
 
+// Publication of a step's result by the last block of the epilogue (as a launch of its own it took a
+// tenth of a step on a small graph).
+struct PrCommit {
+  long long* const* done_ptrs;  // world pointers to every rank's "done" flags; null: nothing is published
+  int world, rank;
+  long long epoch;
+  unsigned int* counter;        // zero before the launch, zero after it
+};
+
 template <int TPR>
 __global__ void __launch_bounds__(256) pagerank_pull_kernel(PrArgs a) {
   const int sub = threadIdx.x % TPR;
@@ -181,11 +190,12 @@ __global__ void __launch_bounds__(256) pagerank_stream_kernel(const long long* r
   }
 }
 
-__global__ void __launch_bounds__(256) pagerank_epilogue_kernel(PrArgs a, const float* acc) {
+__global__ void __launch_bounds__(256) pagerank_epilogue_kernel(PrArgs a, float* acc, int clear, PrCommit c) {
   double dl = 0.0;
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < a.n_local;
        v += (long long)gridDim.x * blockDim.x) {
     const float pr = (1.f - a.damping) + a.damping * acc[v];
+    if (clear) acc[v] = 0.f;
     a.new_contrib[v] = pr * a.inv_outdeg[v];
     if (a.new_rank) {
       if (a.delta_l1) dl += fabs((double)pr - (double)a.old_rank[v]);
@@ -196,21 +206,36 @@ __global__ void __launch_bounds__(256) pagerank_epilogue_kernel(PrArgs a, const 
     dl = pcl_warp_sum_d(dl);
     if ((threadIdx.x & 31) == 0 && dl != 0.0) atomicAdd(a.delta_l1, dl);
   }
+  if (c.done_ptrs == nullptr) return;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(c.counter, 1u) == gridDim.x - 1) {
+    *c.counter = 0u;
+    __threadfence_system();
+    for (int r = 0; r < c.world; ++r) pcl_st_release_sys(c.done_ptrs[r] + c.rank, c.epoch);
+  }
 }
 
 }  // namespace
 
-// Edge-balanced pull step.  `acc` is a scratch vector of n_local floats; it is cleared here.
+// Edge-balanced pull step.  `acc` is a scratch vector of n_local floats: it is cleared here, or, with
+// `acc_clean`, holds zeros on entry and is left with zeros.  With `done_ptrs` the step also publishes
+// `epoch` in every rank's flags once the new contributions are in place (`counter`: one zeroed int).
 // blk_first / blk_last have ceil(nnz / cap) entries (see pagerank_stream_kernel); cap is 2048 or 4096.
 PCL_API int pcl_pagerank_pull_stream(const long long* row_ptr, const int* cols, const float* contrib,
                                      const float* inv_outdeg, long long n_local, long long nnz,
                                      const int* blk_first, const int* blk_last, float damping, float* acc, float* new_contrib, float* new_rank,
-                                     double* delta_l1, const float* old_rank, int cap, cudaStream_t stream) {
-  if (n_local <= 0) return 0;
+                                     double* delta_l1, const float* old_rank, int cap, int acc_clean,
+                                     long long* const* done_ptrs, int world, int rank, long long epoch,
+                                     unsigned int* counter, cudaStream_t stream) {
+  if (n_local <= 0 && done_ptrs == nullptr) return 0;
+  if (n_local < 0) n_local = 0;
   if (cap != 2048 && cap != 4096) return (int)cudaErrorInvalidValue;
   if (delta_l1 != nullptr && (old_rank == nullptr || new_rank == nullptr)) return (int)cudaErrorInvalidValue;
-  cudaError_t e = cudaMemsetAsync(acc, 0, (size_t)n_local * sizeof(float), stream);
-  if (e != cudaSuccess) return (int)e;
+  if (!acc_clean && n_local > 0) {
+    cudaError_t e = cudaMemsetAsync(acc, 0, (size_t)n_local * sizeof(float), stream);
+    if (e != cudaSuccess) return (int)e;
+  }
   if (nnz > 0) {
     long long blocks = (nnz + cap - 1) / cap;
     if (blocks > 148LL * 64) blocks = 148LL * 64;
@@ -222,8 +247,9 @@ PCL_API int pcl_pagerank_pull_stream(const long long* row_ptr, const int* cols, 
   PrArgs a{row_ptr, cols, contrib, inv_outdeg, n_local, damping, new_contrib, new_rank, delta_l1,
            old_rank, 0, nullptr, 0};
   long long eb = (n_local + 255) / 256;
+  if (eb < 1) eb = 1;
   if (eb > 148 * 16) eb = 148 * 16;
-  pagerank_epilogue_kernel<<<(int)eb, 256, 0, stream>>>(a, acc);
+  pagerank_epilogue_kernel<<<(int)eb, 256, 0, stream>>>(a, acc, acc_clean, PrCommit{done_ptrs, world, rank, epoch, counter});
   return pcl_last_error();
 }
 

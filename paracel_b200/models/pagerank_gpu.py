@@ -82,6 +82,10 @@ class PageRankGpu(paralg):
         self.rank_local = torch.where(self.has_out, torch.full_like(od, init), torch.zeros_like(od))
         self.rank_new = torch.empty_like(self.rank_local)
         self.acc = torch.zeros(max(self.n_local, 1), device=dev)
+        # While it stays in the L2, the sums are cleared by the kernel that reads them (20 iterations on 2^17
+        # vertices: 664 us with a memset of its own, 619 us); on 2^24 vertices that took 37 ms instead
+        # of 26 ms, since the cleared sums then push contributions out of the L2.
+        self.acc_clean = self.n_local <= 1 << 21
         self.plan = self._choose_plan()
         # contribution table for iteration 0 lives in tables[0]
         for k in self.KEYS:
@@ -107,7 +111,7 @@ class PageRankGpu(paralg):
                 e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
                 e0.record()
                 pagerank_pull_stream(self.row_ptr, self.cols, probe, self.inv_outdeg, self.d, self.acc,
-                                     out_c, out_r, None, None, plans[cap])
+                                     out_c, out_r, None, None, plans[cap], self.acc_clean)
                 e1.record()
                 torch.cuda.synchronize(dev)
                 times[j] = e0.elapsed_time(e1)
@@ -128,13 +132,13 @@ class PageRankGpu(paralg):
         if self.edge_balanced:
             pagerank_pull_stream(self.row_ptr, self.cols, contrib, self.inv_outdeg, self.d, self.acc,
                                  nxt.shard, self.rank_new, self.delta_l1 if track_delta else None,
-                                 self.rank_local if track_delta else None, self.plan)
+                                 self.rank_local if track_delta else None, self.plan, self.acc_clean, nxt.commit_args())
         else:
             pagerank_pull(self.row_ptr, self.cols, contrib, self.inv_outdeg, self.d,
                           nxt.shard, self.rank_new, self.delta_l1 if track_delta else None,
                           self.rank_local if track_delta else None, self.tpr,
                           self.heavy_rows if self.heavy_rows.numel() else None, self.heavy_deg)
-        self.paracel_commit_write(knxt)
+            self.paracel_commit_write(knxt)
         self.rank_local, self.rank_new = self.rank_new, self.rank_local
         self.it += 1
 

@@ -50,14 +50,14 @@ SIGS = {
     "pcl_gemm_tf32_2sm": "pppiiiqipppppiiiiipiip",
     "pcl_split3_tf32": "ppqiip",
     "pcl_dense_read": "ppqqiipqQpp",
-    "pcl_dense_bupdate": "ppqqiiiffpqQppppp",
+    "pcl_dense_bupdate": "ppqqiiiffppqQppppp",
     "pcl_publish_flag": "piiqp",
     "pcl_dense_push": "ppqqiifp",
     "pcl_validate_ids": "piqqqqpip",
     "pcl_lr_dense_grad": "pppqiipppip",
     "pcl_lr_sparse_grad": "pppppqiippip",
     "pcl_pagerank_pull": "ppppqfppppiqpip",
-    "pcl_pagerank_pull_stream": "ppppqqppfpppppip",
+    "pcl_pagerank_pull_stream": "ppppqqppfpppppiipiiqpp",
     "pcl_lda_gibbs": "ppppppqifffQip",
     "pcl_lda_loglik": "ppppppqifffpp",
     "pcl_als_solve": "ppppppppppqqiiifp",

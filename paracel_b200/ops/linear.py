@@ -67,13 +67,15 @@ def pagerank_stream_plan(row_ptr, cap: int = 2048):
 
 
 def pagerank_pull_stream(row_ptr, cols, contrib, inv_outdeg, damping, acc, new_contrib, new_rank=None,
-                         delta_l1=None, old_rank=None, plan=None):
+                         delta_l1=None, old_rank=None, plan=None, acc_clean: bool = False, commit=None):
     """Edge-balanced pull step: blocks own equal numbers of in-links (good for power-law graphs).
-    ``acc`` is a scratch vector with one float per local vertex; ``plan`` comes from
-    :func:`pagerank_stream_plan` (computed on the fly when missing)."""
+    ``acc`` is a scratch vector with one float per local vertex (``acc_clean``: it holds zeros and is
+    left so); ``plan`` comes from :func:`pagerank_stream_plan` (computed on the fly when missing).
+    ``commit``: ``DenseTable.commit_args()`` of the table that ``new_contrib`` is the shard of; the
+    step then publishes the rewritten shard itself."""
     n = row_ptr.numel() - 1
     if plan is None:
         plan = pagerank_stream_plan(row_ptr)
     _lib.call("pcl_pagerank_pull_stream", row_ptr, cols, contrib, inv_outdeg, n, cols.numel(),
               plan[0], plan[1], float(damping), acc, new_contrib, new_rank, delta_l1, old_rank,
-              int(plan[2]), _lib.stream_ptr())
+              int(plan[2]), int(acc_clean), *(commit or (None, 1, 0, 0, None)), _lib.stream_ptr())

@@ -223,7 +223,6 @@ class DenseTable:
         self.epoch += 1
         b = self.epoch & 1
         s = _lib.stream_ptr()
-        _lib.call("pcl_publish_flag", self._ready_table, self.world, self.rank, self.epoch, s)
         h, reg_lr, reg_lam = _dense_kind(handler or self.handler)
         if lr is None:
             lr = self.lr if reg_lr is None else reg_lr
@@ -232,7 +231,7 @@ class DenseTable:
         if count_nnz:
             self.nnz.zero_()
         _lib.call("pcl_dense_bupdate", self.shard, self._delta_tables[b], self.Lp, self.S, self.world,
-                  self.rank, h, float(lr), float(lam), self.ready, self.epoch, self.timeout_ns,
+                  self.rank, h, float(lr), float(lam), self.ready, self._ready_table, self.epoch, self.timeout_ns,
                   self.status, self._done_table, self.counter, self.nnz if count_nnz else None, s)
 
     def mark_written(self):
@@ -241,6 +240,12 @@ class DenseTable:
         self.epoch += 1
         _lib.call("pcl_publish_flag", self._done_table, self.world, self.rank, self.epoch,
                   _lib.stream_ptr())
+
+    def commit_args(self):
+        """For a kernel that rewrites this rank's shard and publishes the next epoch itself, instead of
+        :meth:`mark_written` behind it: (flag pointers, world, rank, epoch, block counter)."""
+        self.epoch += 1
+        return self._done_table, self.world, self.rank, self.epoch, self.counter
 
     def write(self, values: torch.Tensor):
         """Collective initialisation from a full vector that every rank passes identically: each
