@@ -127,16 +127,10 @@ def available() -> bool:
     return torch.cuda.is_available() and _LIB_PATH.exists()
 
 
-def _conv(a):
-    if a is None:
-        return None
-    if isinstance(a, torch.Tensor):
-        return a.data_ptr()
-    return a
-
-
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current device's current stream (without making a Stream object: that took 7 us,
+    a third of what a launch costs the host)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 _LAUNCHES = 0
@@ -149,9 +143,9 @@ def launches() -> int:
 
 def call(name: str, *args) -> None:
     global _LAUNCHES
-    lib = load()
-    fn = getattr(lib, name)
-    rc = fn(*[_conv(a) for a in args])
+    lib = _LIB if _LIB is not None else load()
+    tensor = torch.Tensor
+    rc = getattr(lib, name)(*[a.data_ptr() if isinstance(a, tensor) else a for a in args])
     _LAUNCHES += 1
     if rc != 0:
         msg = lib.pcl_error_string(rc).decode()
