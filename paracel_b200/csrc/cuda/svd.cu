@@ -181,29 +181,32 @@ int launch_spmm(const long long* row_ptr, const int* cols, const float* vals, lo
 }
 
 // out = M P (TWICE: (M P) P^T) for M [n x K] and P [K x K], K a multiple of 4, fp32 throughout.  A
-// block of 256 threads takes 64 rows at a time: thread (ty, tx) owns rows 4 ty .. 4 ty + 3 and columns
-// tx + 16 j; P and, for the second product, its transpose stay in shared memory, and the product of
-// the first takes the place of the rows there.  Bound by shared-memory loads (4 + 4 KB per 16 KB
-// multiply-adds) at K = 32, where M itself comes out of L2.
+// block of 256 threads takes 128 rows at a time: thread (ty, tx) owns rows ty + 16 i (i < 8) and columns
+// tx + 16 j, sums over even and odd components in the halves of packed multiply-adds.  P^T and, for
+// the second product, P stay in shared memory as rows of components, and the product of the first
+// takes the place of the rows there.  Bound by shared-memory passes: 32 + 4 KB a thread for 64 KB
+// multiply-adds over four components (400 k x 32 and 100 k x 32 twice: 55 us a call on average with 4
+// rows a thread and 4-byte loads of P).
 template <int KB, bool TWICE>
 __global__ void __launch_bounds__(256) rows_times_kernel(const float* __restrict__ M, long long n, int K,
                                                          const float* __restrict__ P, float* __restrict__ out) {
-  constexpr int N = 16 * KB;             // columns, padded with zeros
+  typedef unsigned long long u64;
+  constexpr int N = 16 * KB, R = 128;    // columns padded with zeros; rows of a block
   extern __shared__ __align__(16) float sm[];
-  const int LM = K + 4;
-  float* sP = sm;                        // K x N
-  float* sQ = sP + (TWICE ? K * N : 0);  // K x N: P^T
-  float* sM = sQ + K * N;                // 64 x LM
+  const int LM = K + 4;                  // row pitch: eight rows of sixteen bytes on different banks
+  float* sP = sm;                        // N x LM: column c of P
+  float* sQ = sP + (TWICE ? N * LM : 0); // N x LM: row c of P
+  float* sM = sQ + N * LM;               // R x LM
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   for (int e = tid; e < K * N; e += 256) {
     const int q = e / N, c = e % N;
-    sP[e] = c < K ? __ldg(P + q * K + c) : 0.f;
-    if (TWICE) sQ[e] = c < K ? __ldg(P + c * K + q) : 0.f;
+    sP[c * LM + q] = c < K ? __ldg(P + q * K + c) : 0.f;
+    if (TWICE) sQ[c * LM + q] = c < K ? __ldg(P + c * K + q) : 0.f;
   }
   const int K4 = K / 4;
-  for (long long r0 = (long long)blockIdx.x * 64; r0 < n; r0 += (long long)gridDim.x * 64) {
+  for (long long r0 = (long long)blockIdx.x * R; r0 < n; r0 += (long long)gridDim.x * R) {
     __syncthreads();
-    for (int e = tid; e < 64 * K4; e += 256) {
+    for (int e = tid; e < R * K4; e += 256) {
       const int r = e / K4, c = 4 * (e % K4);
       *reinterpret_cast<float4*>(sM + r * LM + c) =
           r0 + r < n ? __ldg(reinterpret_cast<const float4*>(M + (r0 + r) * K + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -212,38 +215,38 @@ __global__ void __launch_bounds__(256) rows_times_kernel(const float* __restrict
 #pragma unroll
     for (int pass = 0; pass < (TWICE ? 2 : 1); ++pass) {
       const float* B = pass == 0 ? sP : sQ;
-      float acc[4][KB];
+      u64 acc[8][KB];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < KB; ++j) acc[i][j] = 0.f;
-#pragma unroll 2
+        for (int j = 0; j < KB; ++j) acc[i][j] = 0ull;
+#pragma unroll 1
       for (int q = 0; q < K; q += 4) {
-        float4 m[4];
+        ulonglong2 m[8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) m[i] = *reinterpret_cast<const float4*>(sM + (4 * ty + i) * LM + q);
+        for (int i = 0; i < 8; ++i) m[i] = *reinterpret_cast<const ulonglong2*>(sM + (ty + 16 * i) * LM + q);
 #pragma unroll
         for (int j = 0; j < KB; ++j) {
-          const float* b = B + q * N + tx + 16 * j;
-          const float b0 = b[0], b1 = b[N], b2 = b[2 * N], b3 = b[3 * N];
+          const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(B + (tx + 16 * j) * LM + q);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            acc[i][j] = fmaf(m[i].x, b0, acc[i][j]);
-            acc[i][j] = fmaf(m[i].y, b1, acc[i][j]);
-            acc[i][j] = fmaf(m[i].z, b2, acc[i][j]);
-            acc[i][j] = fmaf(m[i].w, b3, acc[i][j]);
+          for (int i = 0; i < 8; ++i) {
+            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][j]) : "l"(m[i].x), "l"(b.x));
+            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][j]) : "l"(m[i].y), "l"(b.y));
           }
         }
       }
       __syncthreads();
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < KB; ++j)
-          if (tx + 16 * j < K) sM[(4 * ty + i) * LM + tx + 16 * j] = acc[i][j];
+        for (int j = 0; j < KB; ++j) {
+          float even, odd;
+          asm("mov.b64 {%0, %1}, %2;" : "=f"(even), "=f"(odd) : "l"(acc[i][j]));
+          if (tx + 16 * j < K) sM[(ty + 16 * i) * LM + tx + 16 * j] = even + odd;
+        }
       __syncthreads();
     }
-    for (int e = tid; e < 64 * K4; e += 256) {
+    for (int e = tid; e < R * K4; e += 256) {
       const int r = e / K4, c = 4 * (e % K4);
       if (r0 + r < n)
         *reinterpret_cast<float4*>(out + (r0 + r) * K + c) = *reinterpret_cast<const float4*>(sM + r * LM + c);
@@ -253,13 +256,13 @@ __global__ void __launch_bounds__(256) rows_times_kernel(const float* __restrict
 
 template <int KB, bool TWICE>
 int launch_rows_times(const float* M, long long n, int K, const float* P, float* out, cudaStream_t stream) {
-  const size_t smem = ((size_t)K * 16 * KB * (TWICE ? 2 : 1) + 64 * (size_t)(K + 4)) * sizeof(float);
+  const size_t smem = (16 * (size_t)KB * (TWICE ? 2 : 1) + 128) * (size_t)(K + 4) * sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(rows_times_kernel<KB, TWICE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rows_times_kernel<KB, TWICE>, 256, smem);
   if (e != cudaSuccess) return (int)e;
-  long long blocks = (n + 63) / 64;
+  long long blocks = (n + 127) / 128;
   const long long most = 148LL * (per_sm > 0 ? per_sm : 1);
   if (blocks > most) blocks = most;
   rows_times_kernel<KB, TWICE><<<(int)blocks, 256, smem, stream>>>(M, n, K, P, out);
@@ -269,20 +272,19 @@ int launch_rows_times(const float* M, long long n, int K, const float* P, float*
 // out[i] = scale * u_i + shift with u_i = (word_i mod 2^24) / 2^24 for the words of the Mersenne Twister
 // MT19937 (Matsumoto and Nishimura, 1998) after init_genrand(seed): the stream of the host
 // generator, made where it is used.
-// One block and one chain of steps.  x[k + 624] = x[k + 397] ^ f(x[k], x[k + 1]) gives 227 words a step;
-// putting the recurrence in for x[k + 397] and again for x[k + 170],
-//   x[k + 624] = x[k - 57] ^ f(x[k - 454], x[k - 453]) ^ f(x[k - 227], x[k - 226]) ^ f(x[k], x[k + 1]),
-// gives 623, and the barrier that ends a step is what a step costs.  The words of a step are tempered
-// and stored under the loads of the next.  3.2 M numbers: 1.54 ms with 227 words a step.
+// One block makes the words, in one chain of steps.  x[k + 624] = x[k + 397] ^ f(x[k], x[k + 1]) gives 227
+// words a step; putting the recurrence in for x[k + 397] and again for x[k + 170] (f is linear),
+//   x[k + 624] = x[k - 57] ^ f(x[k - 454] ^ x[k - 227] ^ x[k], x[k - 453] ^ x[k - 226] ^ x[k + 1]),
+// gives 623, and a step costs little more than the barrier that ends it.  The words are tempered and
+// scaled by a kernel of many blocks behind it.  3.2 M numbers took 1.5 ms with both in one block.
 constexpr int MT_T = 640, MT_W = 623;
 
 __device__ __forceinline__ unsigned mt_f(unsigned a, unsigned b) {
   const unsigned y = (a & 0x80000000u) | (b & 0x7fffffffu);
-  return (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
+  return (y >> 1) ^ ((0u - (y & 1u)) & 0x9908b0dfu);
 }
 
-__global__ void __launch_bounds__(MT_T) mt19937_kernel(float* __restrict__ out, long long n, unsigned seed,
-                                                       float scale, float shift) {
+__global__ void __launch_bounds__(MT_T) mt19937_words_kernel(unsigned* __restrict__ out, long long n, unsigned seed) {
   __shared__ unsigned x[2048];           // word k at k mod 2048: a step reads 1078 back and writes 623
   const int t = threadIdx.x;
   if (t == 0) {
@@ -294,33 +296,35 @@ __global__ void __launch_bounds__(MT_T) mt19937_kernel(float* __restrict__ out, 
     }
   }
   __syncthreads();
-  auto emit = [&](long long i, unsigned v) {
-    v ^= v >> 11;
-    v ^= (v << 7) & 0x9d2c5680u;
-    v ^= (v << 15) & 0xefc60000u;
-    v ^= v >> 18;
-    if (i < n) out[i] = fmaf((float)(v & 0xffffffu) * (1.f / 16777216.f), scale, shift);
-  };
   // words 624 .. 1077 by the recurrence itself: the long form reads 454 words before the state
   for (int k0 = 0; k0 < 454; k0 += 227) {
     if (t < 227) {
       const unsigned v = x[k0 + t + 397] ^ mt_f(x[k0 + t], x[k0 + t + 1]);
       x[k0 + t + 624] = v;
-      emit(k0 + t, v);
+      if (k0 + t < n) out[k0 + t] = v;
     }
     __syncthreads();
   }
-  unsigned last = 0;
-  for (long long i0 = 454; i0 < n + MT_W; i0 += MT_W) {   // the last step only stores
+  for (long long i0 = 454; i0 < n; i0 += MT_W) {
     if (t < MT_W) {
       const int k = (int)((i0 + t) & 2047);
       auto w = [&](int d) { return x[(k + d) & 2047]; };
-      const unsigned a0 = w(-454), a1 = w(-453), b0 = w(-227), b1 = w(-226), c0 = w(0), c1 = w(1), e = w(-57);
-      if (i0 > 454) emit(i0 - MT_W + t, last);
-      last = e ^ mt_f(a0, a1) ^ mt_f(b0, b1) ^ mt_f(c0, c1);
-      x[(k + 624) & 2047] = last;
+      const unsigned v = w(-57) ^ mt_f(w(-454) ^ w(-227) ^ w(0), w(-453) ^ w(-226) ^ w(1));
+      x[(k + 624) & 2047] = v;
+      if (i0 + t < n) out[i0 + t] = v;
     }
     __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(256) mt19937_temper_kernel(float* out, long long n, float scale, float shift) {
+  for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+    unsigned v = __float_as_uint(out[i]);
+    v ^= v >> 11;
+    v ^= (v << 7) & 0x9d2c5680u;
+    v ^= (v << 15) & 0xefc60000u;
+    v ^= v >> 18;
+    out[i] = fmaf((float)(v & 0xffffffu) * (1.f / 16777216.f), scale, shift);
   }
 }
 
@@ -443,7 +447,9 @@ PCL_API int pcl_rows_times(const float* M, long long n, int K, const float* P, i
 PCL_API int pcl_mt19937_uniform(float* out, long long n, unsigned int seed, float scale, float shift,
                                 cudaStream_t stream) {
   if (n <= 0) return 0;
-  mt19937_kernel<<<1, MT_T, 0, stream>>>(out, n, seed, scale, shift);
+  mt19937_words_kernel<<<1, MT_T, 0, stream>>>(reinterpret_cast<unsigned*>(out), n, seed);
+  const long long need = (n + 255) / 256;
+  mt19937_temper_kernel<<<need < 148 * 8 ? (int)need : 148 * 8, 256, 0, stream>>>(out, n, scale, shift);
   return pcl_last_error();
 }
 

@@ -327,11 +327,11 @@ def test_int_row_table_pull_push_match_torch(width, lead):
 
 @pytest.mark.parametrize("K", [4, 12, 16, 20, 32, 52, 100, 112])
 def test_rows_times_matches_fp64(K):
-    """Row counts around a block's 64 rows, columns around the 16 of a thread row."""
+    """Row counts around 64 and a block's 128 rows, columns around the 16 of a thread row."""
     from paracel_b200.ops.svd import rows_times
     g = torch.Generator(device="cuda").manual_seed(K)
     P = torch.randn(K, K, device="cuda", generator=g)
-    for n in (1, 63, 64, 65, 20_011):
+    for n in (1, 63, 64, 65, 127, 128, 129, 20_011):
         M = torch.randn(n, K, device="cuda", generator=g)
         A, P64 = M.double().abs() @ P.double().abs(), P.double()
         u = 2.0 ** -24 * (K + 1)
