@@ -51,6 +51,19 @@ __device__ __forceinline__ void pcl_st_release_sys_i32(int* p, int v) {
   asm volatile("st.release.sys.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// Store `value` in slot [rank] of every rank's flag array, after all that this thread has seen.  A
+// single rank's flags are read by its own GPU only: fences that reach the whole system cost the
+// kernels that publish about 5 us.
+__device__ __forceinline__ void pcl_publish(long long* const* flag_ptrs, int world, int rank, long long value) {
+  if (world == 1) {
+    __threadfence();
+    asm volatile("st.release.gpu.global.s64 [%0], %1;" ::"l"(flag_ptrs[0] + rank), "l"(value) : "memory");
+    return;
+  }
+  __threadfence_system();
+  for (int r = 0; r < world; ++r) pcl_st_release_sys(flag_ptrs[r] + rank, value);
+}
+
 // 128-bit load that bypasses L1 (other SMs / other GPUs may have written it).
 __device__ __forceinline__ float4 pcl_ldcg4(const float* p) {
   float4 v;

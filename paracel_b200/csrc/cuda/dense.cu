@@ -113,18 +113,18 @@ template <bool IS_MAX>
 __global__ void __launch_bounds__(256) dense_bupdate_kernel(BupArgs a) {
   __shared__ int ok;
   // This rank's own "ready": the first block stores it, and waits for nobody before that.
-  if (a.ready_ptrs != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
-    __threadfence_system();
-    for (int r = 0; r < a.world; ++r) pcl_st_release_sys(a.ready_ptrs[r] + a.rank, a.epoch);
-  }
-  if (a.ready != nullptr && a.epoch > 0) {
+  if (a.ready_ptrs != nullptr && blockIdx.x == 0 && threadIdx.x == 0)
+    pcl_publish(a.ready_ptrs, a.world, a.rank, a.epoch);
+  // a single rank's delta was written by earlier work of this stream: nobody to wait for
+  const bool wait = a.world > 1 && a.ready != nullptr && a.epoch > 0;
+  if (wait) {
     if (threadIdx.x == 0)
       ok = pcl_wait_min_clock(a.ready, a.world, a.epoch, a.timeout_ns, a.status, a.rank, 21) ? 1 : 0;
     __syncthreads();
   }
   // After a timed-out wait the block does no work but still takes part in the block count below,
   // so that the counter is back at zero for the next launch; "done" is then not published.
-  const bool proceed = !(a.ready != nullptr && a.epoch > 0) || ok;
+  const bool proceed = !wait || ok;
   const long long lo = (long long)a.rank * a.S;
   long long n = a.L - lo;
   if (n > a.S) n = a.S;
@@ -204,8 +204,7 @@ __global__ void __launch_bounds__(256) dense_bupdate_kernel(BupArgs a) {
     if (prev == gridDim.x - 1) {
       *a.block_counter = 0u;
       if (a.done_ptrs != nullptr && proceed) {
-        __threadfence_system();
-        for (int r = 0; r < a.world; ++r) pcl_st_release_sys(a.done_ptrs[r] + a.rank, a.epoch);
+        pcl_publish(a.done_ptrs, a.world, a.rank, a.epoch);
       }
     }
   }
@@ -251,7 +250,9 @@ __global__ void __launch_bounds__(256) dense_push_kernel(PushDenseArgs a) {
 
 __global__ void publish_kernel(long long* const* flag_ptrs, int world, int rank, long long value) {
   const int r = threadIdx.x;
-  if (r < world) {
+  if (world == 1) {
+    if (r == 0) pcl_publish(flag_ptrs, 1, rank, value);
+  } else if (r < world) {
     __threadfence_system();
     pcl_st_release_sys(flag_ptrs[r] + rank, value);
   }

@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(256) pagerank_heavy_kernel(PrArgs a) {
 // PR_CAP is 2048 or 4096 in-links per block (template parameter).  Which is faster depends on the
 // graph's labelling (R-MAT 26, one GPU: raw labels 6.28 ms with 2048 and 6.04 ms with 4096;
 // block-scrambled labels 7.74 ms and 8.97 ms), so the model times both once at load time.
-constexpr int PR_ROWS = 1024;   // row pointers of a block cached in shared memory up to this many rows
+constexpr int PR_ROWS = 1023;   // row pointers of a block cached in shared memory up to this many rows
 
 // blk_first[b] / blk_last[b]: the rows that contain in-link b * PR_CAP and the last in-link of
 // block b (static per graph, computed once at load time).
@@ -115,6 +115,7 @@ __global__ void __launch_bounds__(256) pagerank_stream_kernel(const long long* r
   __shared__ int srp[PR_ROWS + 1];   // row pointers relative to the block start, clamped to [0, len]
   __shared__ int long_rows[64];
   __shared__ int n_long;
+  __shared__ int cut_first, cut_last;   // the first row begins before the block, the last one ends after it
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (long long blk = blockIdx.x; blk * PR_CAP < nnz; blk += gridDim.x) {
     const long long s = blk * PR_CAP;
@@ -122,8 +123,23 @@ __global__ void __launch_bounds__(256) pagerank_stream_kernel(const long long* r
     const int len = (int)(e - s);
     const long long r0 = blk_first[blk], r1 = blk_last[blk];
     const long long nrows = r1 - r0 + 1;
+    const bool cached = nrows <= PR_ROWS;
     __syncthreads();
-    if (threadIdx.x == 0) n_long = 0;
+    if (threadIdx.x == 0) {
+      n_long = 0;
+      if (!cached) {
+        cut_first = row_ptr[r0] < s;
+        cut_last = row_ptr[r1 + 1] > e;
+      }
+    }
+    // The row pointers are requested with the indices and used behind the gathers: on a small graph a
+    // block is one chain of such latencies.
+    long long rp[(PR_ROWS + 1) / 256];
+#pragma unroll
+    for (int q = 0; q < (PR_ROWS + 1) / 256; ++q) {
+      const int i = threadIdx.x + 256 * q;
+      rp[q] = cached && i <= (int)nrows ? __ldg(row_ptr + r0 + i) : 0;
+    }
     // all index loads of the thread first, then all gathers, then the stores: eight independent
     // random reads in flight per thread instead of a load-use chain per element
 #pragma unroll
@@ -141,14 +157,19 @@ __global__ void __launch_bounds__(256) pagerank_stream_kernel(const long long* r
       for (int q = 0; q < 8; ++q)
         if (ci[q] >= 0) sv[threadIdx.x + (h * 8 + q) * 256] = cv[q];
     }
-    const bool cached = nrows <= PR_ROWS;
     if (cached) {
-      for (int i = threadIdx.x; i <= (int)nrows; i += blockDim.x) {
-        long long v = row_ptr[r0 + i] - s;
+#pragma unroll
+      for (int q = 0; q < (PR_ROWS + 1) / 256; ++q) {
+        const int i = threadIdx.x + 256 * q;
+        if (i > (int)nrows) continue;
+        const long long v = rp[q] - s;
         srp[i] = v < 0 ? 0 : (v > len ? len : (int)v);
+        if (i == 0) cut_first = v < 0;
+        if (i == (int)nrows) cut_last = v > len;
       }
     }
     __syncthreads();
+    auto whole = [&](long long i) { return !(i == 0 && cut_first) && !(i == nrows - 1 && cut_last); };
     // phase A: one thread per row for short segments
     for (long long i = threadIdx.x; i < nrows; i += blockDim.x) {
       int b, en;
@@ -167,8 +188,7 @@ __global__ void __launch_bounds__(256) pagerank_stream_kernel(const long long* r
       float sum = 0.f;
       for (int p = b; p < en; ++p) sum += sv[p];
       const long long r = r0 + i;
-      const bool whole = (i > 0 || row_ptr[r] >= s) && (i < nrows - 1 || row_ptr[r + 1] <= e);
-      if (whole) acc[r] = sum;
+      if (whole(i)) acc[r] = sum;
       else atomicAdd(acc + r, sum);
     }
     __syncthreads();
@@ -177,13 +197,18 @@ __global__ void __launch_bounds__(256) pagerank_stream_kernel(const long long* r
     for (int q = warp; q < nl; q += 8) {
       const long long i = long_rows[q];
       const long long r = r0 + i;
-      const long long rb = row_ptr[r], re = row_ptr[r + 1];
-      const int b = rb > s ? (int)(rb - s) : 0, en = re < e ? (int)(re - s) : len;
+      int b, en;
+      if (cached) { b = srp[i]; en = srp[i + 1]; }
+      else {
+        const long long rb = row_ptr[r], re = row_ptr[r + 1];
+        b = rb > s ? (int)(rb - s) : 0;
+        en = re < e ? (int)(re - s) : len;
+      }
       float sum = 0.f;
       for (int p = b + lane; p < en; p += 32) sum += sv[p];
       sum = pcl_warp_sum(sum);
       if (lane == 0) {
-        if (rb >= s && re <= e) acc[r] = sum;
+        if (whole(i)) acc[r] = sum;
         else atomicAdd(acc + r, sum);
       }
     }
@@ -211,8 +236,7 @@ __global__ void __launch_bounds__(256) pagerank_epilogue_kernel(PrArgs a, float*
   __syncthreads();
   if (threadIdx.x == 0 && atomicAdd(c.counter, 1u) == gridDim.x - 1) {
     *c.counter = 0u;
-    __threadfence_system();
-    for (int r = 0; r < c.world; ++r) pcl_st_release_sys(c.done_ptrs[r] + c.rank, c.epoch);
+    pcl_publish(c.done_ptrs, c.world, c.rank, c.epoch);
   }
 }
 

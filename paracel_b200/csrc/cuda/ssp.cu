@@ -20,7 +20,9 @@ __global__ void ssp_commit_kernel(long long* const* clock_ptrs, int world, int r
   // a rank whose wait ran out (or that met a bad id) this round does not announce progress
   if (pcl_status_code(status) != 0) return;
   int r = threadIdx.x;
-  if (r < world) {
+  if (world == 1) {
+    if (r == 0) pcl_publish(clock_ptrs, 1, rank, value);
+  } else if (r < world) {
     __threadfence_system();  // order this rank's earlier pushes before the clock
     pcl_st_release_sys(clock_ptrs[r] + rank, value);
   }
