@@ -243,8 +243,13 @@ __device__ __forceinline__ float sg_residual(const SparseGradArgs& a, float z, f
   return r;
 }
 
-__device__ __forceinline__ void sg_scatter(const SparseGradArgs& a, int* s_hot, int c, float t, bool fx_ok) {
-  if (c < a.hot_T && fx_ok && fabsf(t) < 64.f) atomicAdd(&s_hot[c], __float2int_rn(t * SG_FX));
+// FX: fixed point.  Squared-loss residuals are unbounded and keep floating-point sums (in shared memory
+// too: sent straight to global memory, the additions to the hottest features queued up at a few
+// addresses and took six times as long as everything else).
+template <bool FX>
+__device__ __forceinline__ void sg_scatter(const SparseGradArgs& a, int* s_hot, int c, float t) {
+  if (!FX && c < a.hot_T) atomicAdd(reinterpret_cast<float*>(s_hot) + c, t);
+  else if (FX && c < a.hot_T && fabsf(t) < 64.f) atomicAdd(&s_hot[c], __float2int_rn(t * SG_FX));
   else atomicAdd(a.g + c, t);
 }
 
@@ -253,78 +258,112 @@ __device__ __forceinline__ void sg_scatter(const SparseGradArgs& a, int* s_hot, 
 // only as many chains in flight as resident warps (long scoreboard 17 stall cycles per issue).
 // Rows of up to 64 non-zeros keep their ids and values in registers between the margin and the
 // scatter; longer rows take the loop form.
-// Measured on 50 M x 2^24 with 40 non-zeros per row: 1 / 2 / 4 / 8 rows per step give 2.04 / 3.16 /
-// 3.36 / 2.06 G samples/s (eight rows cost too many registers).
-__global__ void __launch_bounds__(256) sparse_grad_kernel(SparseGradArgs a) {
+// Measured on 50 M x 2^24 with 40 non-zeros per row: 1 / 2 / 4 / 8 rows per step gave 2.04 / 3.16 /
+// 3.36 / 2.06 G samples/s (eight rows cost too many registers).  The stream (limits, ids, values) is read
+// one step ahead and past the caches' stock of weights: an epoch over 8 M such rows, four
+// minibatches, 2483 -> 2121 us; 2 M rows of 20 values 527 -> 399 us.  Three CTAs per SM without the few
+// spilled registers, or two rows per step with five CTAs, gave 2280 us.
+template <bool VALS, bool FX>
+__global__ void __launch_bounds__(256, 4) sparse_grad_kernel(SparseGradArgs a) {
   extern __shared__ int s_hot[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   for (int j = threadIdx.x; j < a.hot_T; j += blockDim.x) s_hot[j] = 0;
   __syncthreads();
   double loss = 0.0;
-  // squared-loss residuals are unbounded: keep those in floating point
-  const bool fx_ok = a.logistic != 0;
   const long long stride = (long long)gridDim.x * wpb;
-  for (long long row0 = (long long)blockIdx.x * wpb + warp; row0 < a.n; row0 += SG_ROWS * stride) {
-    long long rb[SG_ROWS], re[SG_ROWS];
-    bool shortrows = true;
+  // limits of a step's rows and ids and values of short rows, read one step ahead
+  long long rb[SG_ROWS];
+  int len[SG_ROWS], c[2 * SG_ROWS];
+  float v[VALS ? 2 * SG_ROWS : 1];
+  long long nb[SG_ROWS], ne[SG_ROWS];
+  auto limits = [&](long long row0) {
 #pragma unroll
     for (int k = 0; k < SG_ROWS; ++k) {
       const long long row = row0 + k * stride;
       const bool has = row < a.n;
-      rb[k] = has ? a.row_ptr[row] : 0;
-      re[k] = has ? a.row_ptr[row + 1] : 0;
-      shortrows &= (re[k] - rb[k] <= 64);
+      nb[k] = has ? __ldg(a.row_ptr + row) : 0;
+      ne[k] = has ? __ldg(a.row_ptr + row + 1) : 0;
     }
-    if (shortrows) {
-      // ids and values of all rows, then all gathers, then the reductions
-      int c[2 * SG_ROWS];
-      float v[2 * SG_ROWS], t[2 * SG_ROWS];
+  };
+  auto entries = [&]() {
 #pragma unroll
-      for (int q = 0; q < 2 * SG_ROWS; ++q) {
-        const long long p = rb[q >> 1] + (q & 1) * 32 + lane;
-        const bool in = p < re[q >> 1];
-        c[q] = in ? __ldg(a.cols + p) : -1;
-        v[q] = (in && a.vals) ? __ldg(a.vals + p) : 1.f;
-      }
+    for (int k = 0; k < SG_ROWS; ++k) {
+      rb[k] = nb[k];
+      len[k] = (int)(ne[k] - nb[k]);
+    }
+#pragma unroll
+    for (int q = 0; q < 2 * SG_ROWS; ++q) {
+      const int i = (q & 1) * 32 + lane;
+      const bool in = i < len[q >> 1];
+      c[q] = in ? __ldcs(a.cols + rb[q >> 1] + i) : -1;
+      if (VALS) v[VALS ? q : 0] = in ? __ldcs(a.vals + rb[q >> 1] + i) : 1.f;
+    }
+  };
+  long long row0 = (long long)blockIdx.x * wpb + warp;
+  if (row0 < a.n) {
+    limits(row0);
+    entries();
+  }
+  for (; row0 < a.n; row0 += SG_ROWS * stride) {
+    const long long next = row0 + SG_ROWS * stride;
+    limits(next);                                // rows past the end: empty
+    bool shortrows = true;
+#pragma unroll
+    for (int k = 0; k < SG_ROWS; ++k) shortrows &= len[k] <= 64;
+    if (shortrows) {
+      float t[2 * SG_ROWS];
 #pragma unroll
       for (int q = 0; q < 2 * SG_ROWS; ++q) t[q] = c[q] >= 0 ? __ldg(a.theta + c[q]) : 0.f;
+      float yy[SG_ROWS];
+#pragma unroll
+      for (int k = 0; k < SG_ROWS; ++k) yy[k] = row0 + k * stride < a.n ? __ldcs(a.y + row0 + k * stride) : 0.f;
+      int c0[2 * SG_ROWS];
+      float v0[VALS ? 2 * SG_ROWS : 1];
+#pragma unroll
+      for (int q = 0; q < 2 * SG_ROWS; ++q) {
+        c0[q] = c[q];
+        if (VALS) v0[VALS ? q : 0] = v[VALS ? q : 0];
+      }
+      entries();
       float z[SG_ROWS];
 #pragma unroll
-      for (int k = 0; k < SG_ROWS; ++k) z[k] = fmaf(v[2 * k], t[2 * k], v[2 * k + 1] * t[2 * k + 1]);
+      for (int k = 0; k < SG_ROWS; ++k)
+        z[k] = VALS ? fmaf(v0[VALS ? 2 * k : 0], t[2 * k], v0[VALS ? 2 * k + 1 : 0] * t[2 * k + 1]) : t[2 * k] + t[2 * k + 1];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
         for (int k = 0; k < SG_ROWS; ++k) z[k] += __shfl_xor_sync(0xffffffffu, z[k], o);
 #pragma unroll
       for (int k = 0; k < SG_ROWS; ++k) {
-        const long long row = row0 + k * stride;
-        if (row >= a.n) break;
-        const float r = sg_residual(a, z[k], a.y[row], loss);
-        if (c[2 * k] >= 0) sg_scatter(a, s_hot, c[2 * k], r * v[2 * k], fx_ok);
-        if (c[2 * k + 1] >= 0) sg_scatter(a, s_hot, c[2 * k + 1], r * v[2 * k + 1], fx_ok);
+        if (row0 + k * stride >= a.n) break;
+        const float r = sg_residual(a, z[k], yy[k], loss);
+        if (c0[2 * k] >= 0) sg_scatter<FX>(a, s_hot, c0[2 * k], VALS ? r * v0[VALS ? 2 * k : 0] : r);
+        if (c0[2 * k + 1] >= 0) sg_scatter<FX>(a, s_hot, c0[2 * k + 1], VALS ? r * v0[VALS ? 2 * k + 1 : 0] : r);
       }
       continue;
     }
     for (int k = 0; k < SG_ROWS; ++k) {
       const long long row = row0 + k * stride;
       if (row >= a.n) break;
+      const long long b = rb[k], e = b + len[k];
       float zz = 0.f;
-      for (long long q = rb[k] + lane; q < re[k]; q += 32) {
-        const float vv = a.vals ? a.vals[q] : 1.f;
+      for (long long q = b + lane; q < e; q += 32) {
+        const float vv = VALS ? a.vals[q] : 1.f;
         zz = fmaf(vv, __ldg(a.theta + a.cols[q]), zz);
       }
       zz = pcl_warp_sum(zz);
       const float r = sg_residual(a, zz, a.y[row], loss);
-      for (long long q = rb[k] + lane; q < re[k]; q += 32) {
-        const float vv = a.vals ? a.vals[q] : 1.f;
-        sg_scatter(a, s_hot, a.cols[q], r * vv, fx_ok);
+      for (long long q = b + lane; q < e; q += 32) {
+        const float vv = VALS ? a.vals[q] : 1.f;
+        sg_scatter<FX>(a, s_hot, a.cols[q], r * vv);
       }
     }
+    entries();
   }
   __syncthreads();
   for (int j = threadIdx.x; j < a.hot_T; j += blockDim.x) {
-    const int v = s_hot[j];
-    if (v != 0) atomicAdd(a.g + j, (float)v * SG_FXI);
+    const float v = FX ? (float)s_hot[j] * SG_FXI : __int_as_float(s_hot[j]);
+    if (v != 0.f) atomicAdd(a.g + j, v);
   }
   if (lane == 0 && loss != 0.0) atomicAdd(a.loss, loss);
 }
@@ -393,20 +432,22 @@ PCL_API int pcl_lr_sparse_grad(const long long* row_ptr, const int* cols, const 
   if (hot_T < 0 || hot_T > 24 * 1024) return (int)cudaErrorInvalidValue;
   SparseGradArgs a{row_ptr, cols, vals, y, theta, n, logistic, hot_T, g, loss};
   size_t smem = (size_t)hot_T * sizeof(float);
-  cudaError_t e = cudaFuncSetAttribute(sparse_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  auto kernel = vals != nullptr ? (logistic ? sparse_grad_kernel<true, true> : sparse_grad_kernel<true, false>)
+                                : (logistic ? sparse_grad_kernel<false, true> : sparse_grad_kernel<false, false>);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
   if (e != cudaSuccess) return (int)e;
   if (blocks <= 0) {
     // as many blocks as are resident at once (the kernel is bound by gather / atomic latency,
     // so every resident warp counts; the shared-memory table of hot features sets the limit)
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sparse_grad_kernel, 256, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, smem);
     if (e != cudaSuccess) return (int)e;
     blocks = 148 * (per_sm > 0 ? per_sm : 4);
   }
   long long need = (n + 7) / 8;
   if (need < blocks) blocks = (int)need;
-  sparse_grad_kernel<<<blocks, 256, smem, stream>>>(a);
+  kernel<<<blocks, 256, smem, stream>>>(a);
   return pcl_last_error();
 }
 

@@ -253,3 +253,40 @@ def test_dense_gradient_at_the_edges_of_its_row_kernels(d):
             bound = X64.abs().T @ dr + (n + 2) * 2.0 ** -24 * (X64.abs().T @ r.abs())
             assert bool(((grad.double() - X64.T @ r).abs() <= bound).all()), (n, lead)
             assert abs(float(loss) - float((r * r).sum())) <= float((2 * r.abs() * dr + dr * dr).sum()) + 1e-12
+
+
+@pytest.mark.parametrize("n,F", [(1, 3), (5, 7), (40, 9000), (90_000, 20_000)])
+@pytest.mark.parametrize("logistic", [True, False])
+@pytest.mark.parametrize("valued", [True, False])
+def test_sparse_gradient_read_one_step_ahead(n, F, logistic, valued):
+    """Rows of 0 to 70 entries (the register form takes 64), steps that end past the last row, one block
+    and many, fewer features than the hot table holds, values up to 12."""
+    from paracel_b200.ops.linear import sparse_grad
+    g = torch.Generator(device="cuda").manual_seed(n)
+    lens = torch.randint(0, 12, (n,), device="cuda", generator=g)
+    lens[n // 2] = 70
+    if n > 100:
+        lens[100], lens[-1] = 64, 65
+    ptr = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+    ptr[1:] = lens.cumsum(0)
+    nnz = int(ptr[-1])
+    cols = (torch.rand(nnz, device="cuda", generator=g) ** 4 * F).int().clamp(max=F - 1)
+    vals = 12 * torch.rand(nnz, device="cuda", generator=g) if valued else None
+    v64 = vals.double() if valued else torch.ones(nnz, device="cuda").double()
+    theta = 0.05 * torch.randn(F, device="cuda", generator=g)
+    y = (torch.rand(n, device="cuda", generator=g) < 0.5).float()
+    row = torch.repeat_interleave(torch.arange(n, device="cuda"), lens)
+    zero = torch.zeros(n, dtype=torch.float64, device="cuda")
+    z = zero.index_add(0, row, v64 * theta.double()[cols.long()])
+    zmag = zero.index_add(0, row, v64 * theta.double()[cols.long()].abs())
+    r = y.double() - (torch.sigmoid(z) if logistic else z)
+    fzero = torch.zeros(F, dtype=torch.float64, device="cuda")
+    ref = fzero.index_add(0, cols.long(), r[row] * v64)
+    mag = fzero.index_add(0, cols.long(), v64 * (1 + zmag[row]))
+    cnt = torch.bincount(cols.long(), minlength=F).double()
+    for blocks in (0, 1):
+        grad, loss = torch.zeros(F, device="cuda"), torch.zeros(1, dtype=torch.float64, device="cuda")
+        sparse_grad(ptr, cols, vals, y, theta, grad, loss, logistic=logistic, blocks=blocks)
+        # half a unit of the fixed-point table per term; margins of up to 70 terms; fp32 sums of cnt terms
+        bound = (cnt * 2.0 ** -15 if logistic else 0) + (cnt + 90) * 2.0 ** -23 * mag
+        assert bool(((grad.double() - ref).abs() <= bound + 1e-30).all())
