@@ -69,6 +69,87 @@ __global__ void __launch_bounds__(256) kmeans_accumulate_vec_kernel(const float*
   }
 }
 
+// Few clusters: the reductions above all go to a few addresses (900 k points of 8 columns in 10 clusters
+// took 1.19 ms, now 13 us; of 100 columns in 12 clusters 1.41 ms, now 70 us).  Here every group of LG lanes that takes a
+// point at a time has sums of its own in shared memory, plain additions without atomics, and a block
+// adds its copies up at the end.  A lane owns PIECES 16-byte pieces of a row; four points are in
+// flight per group.
+template <int LG, int PIECES>
+__global__ void kmeans_accumulate_few_kernel(const float* X, const int* assign, long long n, int d, int k,
+                                             int copy_floats, float* sums, float* counts) {
+  constexpr int U = 4;
+  extern __shared__ __align__(16) float s_c[];     // copies x (k x d sums, k counts)
+  const int groups = blockDim.x / LG, grp = threadIdx.x / LG, l = threadIdx.x % LG;
+  for (int e = threadIdx.x; e < groups * copy_floats; e += blockDim.x) s_c[e] = 0.f;
+  __syncthreads();
+  float* mine = s_c + grp * copy_floats;
+  const long long step = (long long)gridDim.x * groups;
+  for (long long i0 = (long long)blockIdx.x * groups + grp; i0 < n; i0 += U * step) {
+    int c[U];
+    float4 x[U][PIECES];
+#pragma unroll
+    for (int u = 0; u < U; ++u) c[u] = i0 + u * step < n ? __ldg(assign + i0 + u * step) : -1;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int q = 0; q < PIECES; ++q) {
+        const int j = 4 * (q * LG + l);
+        if (i0 + u * step < n && j < d) x[u][q] = __ldcs(reinterpret_cast<const float4*>(X + (i0 + u * step) * d + j));
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (c[u] < 0 || c[u] >= k) continue;
+#pragma unroll
+      for (int q = 0; q < PIECES; ++q) {
+        const int j = 4 * (q * LG + l);
+        if (j < d) {
+          float4* p = reinterpret_cast<float4*>(mine + c[u] * d + j);
+          float4 v = *p;
+          v.x += x[u][q].x; v.y += x[u][q].y; v.z += x[u][q].z; v.w += x[u][q].w;
+          *p = v;
+        }
+      }
+      if (l == 0) mine[k * d + c[u]] += 1.f;
+    }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < k * d + k; e += blockDim.x) {
+    float v = 0.f;
+    for (int g = 0; g < groups; ++g) v += s_c[g * copy_floats + e];
+    if (v != 0.f) atomicAdd(e < k * d ? sums + e : counts + (e - k * d), v);
+  }
+}
+
+// Warps of a block of kmeans_accumulate_few_kernel; 0: the clusters are too many.  Six groups per SM beat
+// the reductions (500 k points: 64 columns in 100 clusters 235 -> 171 us, 128 in 64 362 -> 174 us),
+// three did not (128 in 120: 324 against 336 us).
+inline int km_few_warps(long long copy_bytes, int groups_per_warp) {
+  if (copy_bytes <= 100 * 1024 / 3) return (int)(100 * 1024 / copy_bytes < 8 ? 100 * 1024 / copy_bytes : 8);
+  const int w = (int)(200 * 1024 / copy_bytes);
+  return w * groups_per_warp >= 5 ? w : 0;
+}
+
+template <int LG, int PIECES>
+int launch_km_few(const float* X, const int* assign, long long n, int d, int k, float* sums, float* counts,
+                  bool* taken, cudaStream_t stream) {
+  const long long copy_floats = ((long long)k * (d + 1) + 3) / 4 * 4;
+  const int warps = km_few_warps(copy_floats * 4 * (32 / LG), 32 / LG);
+  *taken = warps > 0;
+  if (warps == 0) return 0;
+  auto kernel = kmeans_accumulate_few_kernel<LG, PIECES>;
+  const size_t smem = (size_t)copy_floats * 4 * (32 / LG) * warps;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  int per_sm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * warps, smem);
+  if (e != cudaSuccess) return (int)e;
+  const long long per_block = (long long)warps * (32 / LG) * 4;
+  long long blocks = (n + per_block - 1) / per_block;
+  if (blocks > 148LL * (per_sm > 0 ? per_sm : 1)) blocks = 148LL * (per_sm > 0 ? per_sm : 1);
+  kernel<<<(int)blocks, 32 * warps, smem, stream>>>(X, assign, n, d, k, (int)copy_floats, sums, counts);
+  return pcl_last_error();
+}
+
 // Lane i of the warp holds the i-th best (value, id) of its row, best first.  Bound by reading S
 // once: a warp asks for TK_U x 128 columns before it looks at the first (2 KB in flight per warp, with
 // 32 columns at a time the scan of a row was a chain of load latencies), and the 8-byte column ids,
@@ -323,12 +404,25 @@ __global__ void __launch_bounds__(256) allreduce_sum_kernel(ArArgs a) {
 
 }  // namespace
 
-PCL_API int pcl_kmeans_accumulate(const float* X, const int* assign, long long n, int d, float* sums,
+PCL_API int pcl_kmeans_accumulate(const float* X, const int* assign, long long n, int d, int k, float* sums,
                                   float* counts, cudaStream_t stream) {
   if (n <= 0) return 0;
   long long blocks = (n + 7) / 8;
   if (blocks > 148 * 8) blocks = 148 * 8;
   const bool vec = (d % 4 == 0) && d <= 512 && (((uintptr_t)X | (uintptr_t)sums) & 15) == 0;
+  if (vec && k > 0) {
+    bool taken = false;
+    int rc;
+    if (d <= 4) rc = launch_km_few<1, 1>(X, assign, n, d, k, sums, counts, &taken, stream);
+    else if (d <= 8) rc = launch_km_few<2, 1>(X, assign, n, d, k, sums, counts, &taken, stream);
+    else if (d <= 16) rc = launch_km_few<4, 1>(X, assign, n, d, k, sums, counts, &taken, stream);
+    else if (d <= 32) rc = launch_km_few<8, 1>(X, assign, n, d, k, sums, counts, &taken, stream);
+    else if (d <= 64) rc = launch_km_few<16, 1>(X, assign, n, d, k, sums, counts, &taken, stream);
+    else if (d <= 128) rc = launch_km_few<32, 1>(X, assign, n, d, k, sums, counts, &taken, stream);
+    else if (d <= 256) rc = launch_km_few<32, 2>(X, assign, n, d, k, sums, counts, &taken, stream);
+    else rc = launch_km_few<32, 4>(X, assign, n, d, k, sums, counts, &taken, stream);
+    if (rc != 0 || taken) return rc;
+  }
   if (vec) {
     blocks = (n + 31) / 32;
     if (blocks > 148 * 8) blocks = 148 * 8;

@@ -61,7 +61,7 @@ SIGS = {
     "pcl_lda_gibbs": "ppppppqifffQip",
     "pcl_lda_loglik": "ppppppqifffpp",
     "pcl_als_solve": "ppppppppppqqiiifp",
-    "pcl_kmeans_accumulate": "ppqippp",
+    "pcl_kmeans_accumulate": "ppqiippp",
     "pcl_topk_rows": "pqiippfippp",
     "pcl_balltree_search": "pppppppiiipppp",
     "pcl_partition_count": "ppqiipp",

@@ -13,7 +13,8 @@ def kmeans_accumulate(X: torch.Tensor, assign: torch.Tensor, sums: torch.Tensor,
     """sums[c] += X[i], counts[c] += 1 for c = assign[i]."""
     _lib.check_cuda(X, torch.float32, "X")
     _lib.check_cuda(assign, torch.int32, "assign")
-    _lib.call("pcl_kmeans_accumulate", X, assign, X.shape[0], X.shape[1], sums, counts, _lib.stream_ptr())
+    _lib.call("pcl_kmeans_accumulate", X, assign, X.shape[0], X.shape[1], counts.numel(), sums, counts,
+              _lib.stream_ptr())
 
 
 class RunningTopK:

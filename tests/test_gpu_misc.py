@@ -350,3 +350,22 @@ def test_host_rand_is_the_cpu_generators_stream(n, seed):
     ref = torch.rand(n, generator=g)
     assert torch.equal(host_rand((n,), seed, "cuda").cpu(), ref)
     assert torch.equal(host_rand((n,), seed, "cuda", 2.0, -1.0).cpu(), ref * 2 - 1)
+
+
+@pytest.mark.parametrize("d,k", [(4, 1), (4, 3000), (8, 10), (12, 30), (20, 7), (36, 100), (64, 100), (64, 900), (100, 12),
+                                 (128, 2), (128, 130), (200, 40), (512, 8)])
+def test_kmeans_accumulate_with_few_clusters(d, k):
+    """Every group width, on both sides of the limit by which a block keeps its own sums; clusters that
+    nobody is in, fewer points than groups."""
+    from paracel_b200.ops.misc import kmeans_accumulate
+    g = torch.Generator(device="cuda").manual_seed(d * k)
+    for n in (1, 5, 1003, 60_001):
+        X = torch.randn(n, d, device="cuda", generator=g)
+        a = (torch.rand(n, device="cuda", generator=g) ** 2 * k).int().clamp(max=k - 1)
+        sums, counts = torch.ones(k, d, device="cuda"), torch.ones(k, device="cuda")
+        kmeans_accumulate(X, a, sums, counts)
+        ref = torch.ones(k, d, dtype=torch.float64, device="cuda").index_add_(0, a.long(), X.double())
+        mag = torch.ones(k, d, dtype=torch.float64, device="cuda").index_add_(0, a.long(), X.double().abs())
+        cnt = 1 + torch.bincount(a.long(), minlength=k).double()
+        assert torch.equal(counts.double(), cnt)
+        assert bool(((sums.double() - ref).abs() <= (cnt[:, None] + 1) * 2.0 ** -24 * mag).all())
