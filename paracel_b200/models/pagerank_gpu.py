@@ -82,10 +82,10 @@ class PageRankGpu(paralg):
         self.rank_local = torch.where(self.has_out, torch.full_like(od, init), torch.zeros_like(od))
         self.rank_new = torch.empty_like(self.rank_local)
         self.acc = torch.zeros(max(self.n_local, 1), device=dev)
-        # While it stays in the L2, the sums are cleared by the kernel that reads them (20 iterations on 2^17
-        # vertices: 664 us with a memset of its own, 619 us); on 2^24 vertices that took 37 ms instead
-        # of 26 ms, since the cleared sums then push contributions out of the L2.
-        self.acc_clean = self.n_local <= 1 << 21
+        # On small graphs the kernel that reads the sums clears them, which saves a launch (20 iterations on
+        # 2^14 vertices: 435 -> 411 us; on 2^17: 529 -> 517 us).  From 2^18 on a memset of its own is faster
+        # (2^18: 693 -> 625 us, 2^22: 6.6 -> 3.8 ms).
+        self.acc_clean = self.n_local <= 1 << 17
         self.plan = self._choose_plan()
         # contribution table for iteration 0 lives in tables[0]
         for k in self.KEYS:
