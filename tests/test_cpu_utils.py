@@ -319,3 +319,10 @@ def test_topk_lists_ends_a_row_at_its_first_empty_slot(m, k):
         idx[r, n[r]:] = -1
     exp = {int(ids[r]): [(int(idx[r, j]), float(val[r, j])) for j in range(n[r])] for r in range(m) if n[r]}
     assert core().topk_lists(ids, idx, val) == exp
+
+
+def test_topk_lists_skips_negative_ids_between_others():
+    """Column ids are the caller's and may be negative: such a slot is left out, those behind it stay."""
+    idx = np.array([[4, -3, 9, -1], [-7, -1, -1, -1], [-2, 5, -1, -1]])
+    val = np.arange(12, dtype=np.float32).reshape(3, 4)
+    assert core().topk_lists(np.array([10, 20, -30]), idx, val) == {10: [(4, 0.0), (9, 2.0)], -30: [(5, 9.0)]}
