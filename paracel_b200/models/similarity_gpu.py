@@ -54,7 +54,6 @@ class SimDenseGpu(paralg):
             dist.all_gather(allnb, nb, group=self.group)
         counts = [int(x.item()) for x in allnb]
         self.rps = max(max(counts), 1)                    # common block height
-        self.padded = any(c < self.rps for c in counts)   # some block ends in padding rows
         # ids of every row of the gathered matrix (-1 marks padding rows)
         mine = torch.full((self.rps,), -1, dtype=torch.int64, device=dev)
         mine[: B.shape[0]] = ids_b.to(dev, torch.int64)
@@ -64,6 +63,7 @@ class SimDenseGpu(paralg):
         else:
             parts = [mine]
         self.ids_b_all = torch.cat(parts).contiguous()
+        self.masked = bool((self.ids_b_all < 0).any())    # padding rows, or negative ids of the caller's
         self.tab = self.paracel_matrix_table("sim_block", self.rps * self.world, 3 * self.dp)
         Bn = torch.zeros(self.rps, self.dp, device=dev)
         Bn[: B.shape[0], : self.d] = self._normalise(B.to(dev, torch.float32))
@@ -80,8 +80,8 @@ class SimDenseGpu(paralg):
         for r0 in range(0, m, self.chunk_rows):
             r1 = min(m, r0 + self.chunk_rows)
             St = self.paracel_read_matmul("sim_block", split3(self.A[r0:r1].contiguous(), False), S[: r1 - r0])
-            if self.padded:
-                St[:, self.ids_b_all < 0] = -3.0e38       # padding rows carry id -1
+            if self.masked:
+                St[:, self.ids_b_all < 0] = -3.0e38       # nobody's neighbours
             part = RunningTopK(self.ids_a[r0:r1], self.ktop, self.simbar)
             part.update(St, self.ids_b_all)
             topk.val[r0:r1], topk.idx[r0:r1] = part.val, part.idx

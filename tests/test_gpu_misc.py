@@ -369,3 +369,24 @@ def test_kmeans_accumulate_with_few_clusters(d, k):
         cnt = 1 + torch.bincount(a.long(), minlength=k).double()
         assert torch.equal(counts.double(), cnt)
         assert bool(((sums.double() - ref).abs() <= (cnt[:, None] + 1) * 2.0 ** -24 * mag).all())
+
+
+def test_similarity_leaves_out_rows_with_negative_ids():
+    """A row of B with a negative id is nobody's neighbour and takes no place among the ktop."""
+    from paracel_b200.models.similarity_gpu import SimDenseGpu
+    g = torch.Generator(device="cuda").manual_seed(5)
+    n, d, top = 60, 12, 4
+    ids = torch.arange(n, device="cuda")
+    ids[::3] = -1 - ids[::3]
+    X = torch.randn(n, d, device="cuda", generator=g)
+    m = SimDenseGpu(d, ktop=top, simbar=-1.0, device="cuda")
+    m.load(ids, X)
+    m.solve()
+    Xn = X.double() / X.double().norm(dim=1, keepdim=True)
+    S = Xn @ Xn.T
+    S[:, ids < 0] = -9.0
+    S.fill_diagonal_(-9.0)
+    order = torch.sort(S, dim=1, descending=True).indices[:, :top]
+    assert {r: [c for c, _ in v] for r, v in m.result.items()} == {
+        int(ids[r]): [int(ids[c]) for c in order[r]] for r in range(n)}
+    m.free()
