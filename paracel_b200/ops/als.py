@@ -19,6 +19,9 @@ def als_solve(user_ptr: torch.Tensor, item_idx: torch.Tensor, rating: torch.Tens
     of H) and ``rating`` (fp32).  Users with more than ``seg_len`` ratings are split over
     several CTAs.  Returns W [n_users, k]."""
     dev = H.device
+    for name, t in (("user_ptr", user_ptr), ("item_idx", item_idx), ("rating", rating)):
+        if t.device != dev:                   # their addresses go to the kernels as they are
+            raise ValueError(f"{name} is on {t.device}, H on {dev}")
     H = H.contiguous().float()
     n_users, k = user_ptr.numel() - 1, H.shape[1]
     # the kernel gathers rows of H by these indices without looking at them again

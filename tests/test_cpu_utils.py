@@ -326,3 +326,14 @@ def test_topk_lists_skips_negative_ids_between_others():
     idx = np.array([[4, -3, 9, -1], [-7, -1, -1, -1], [-2, 5, -1, -1]])
     val = np.arange(12, dtype=np.float32).reshape(3, 4)
     assert core().topk_lists(np.array([10, 20, -30]), idx, val) == {10: [(4, 0.0), (9, 2.0)], -30: [(5, 9.0)]}
+
+
+@pytest.mark.parametrize("away", ["user_ptr", "item_idx", "rating"])
+def test_als_solve_refuses_arrays_off_the_factors_device(away):
+    """The kernels take raw addresses, so an array on another device than H is refused on the host."""
+    import torch
+    from paracel_b200.ops.als import als_solve
+    args = {"user_ptr": torch.tensor([0, 1]), "item_idx": torch.zeros(1, dtype=torch.int32), "rating": torch.ones(1)}
+    args = {k: v if k == away else v.to("meta") for k, v in args.items()}
+    with pytest.raises(ValueError, match=away):
+        als_solve(H=torch.zeros(4, 8, device="meta"), lam=0.1, **args)
