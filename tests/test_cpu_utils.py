@@ -337,3 +337,11 @@ def test_als_solve_refuses_arrays_off_the_factors_device(away):
     args = {k: v if k == away else v.to("meta") for k, v in args.items()}
     with pytest.raises(ValueError, match=away):
         als_solve(H=torch.zeros(4, 8, device="meta"), lam=0.1, **args)
+
+
+@pytest.mark.parametrize("seed,device,what", [(1 << 64, "cuda", "Overflow"), (1.5, "cuda", "manual_seed"),
+                                              (None, "cuda", "manual_seed"), (3, "cpu", "CUDA device")])
+def test_host_rand_refuses_what_the_host_generator_refuses(seed, device, what):
+    from paracel_b200.ops.svd import host_rand
+    with pytest.raises((ValueError, RuntimeError), match=what):
+        host_rand((4,), seed, device)
