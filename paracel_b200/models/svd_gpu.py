@@ -11,7 +11,8 @@ writes its part into ``paracel_delta_buffer(key)`` and a collective ``paracel_bu
 sum.  Stage 2 is the Cholesky-QR of W and H (``M^T M = R^T R``, ``Q = M R^-1``) and the SVD of the
 K x K matrix ``R_W R_H^T`` (on the host, svd.hpp:294-298), ``U = Q_W U_r``, ``V = Q_H V_r``.
 
-Kernels: CSR products ``A.H`` / ``A^T.W`` (the second on a transposed copy of A made by ``load``),
+Kernels: CSR products ``A.H`` / ``A^T.W`` (the second on a transposed copy of A made by ``load``, or by
+scattered additions where the matrix is too large for a copy),
 products of a tall matrix with a K x K one and the small Cholesky factor (csrc/cuda/svd.cu), and the
 Gram matrix (``pcl_gram``)."""
 from __future__ import annotations
@@ -21,7 +22,7 @@ import os
 import torch
 
 from ..ops.misc import gram
-from ..ops.svd import chol_factor, host_rand, rows_times, spmm_csr
+from ..ops.svd import chol_factor, host_rand, rows_times, spmm_csr, spmm_csr_t
 from ..paralg import paralg
 
 
@@ -34,6 +35,13 @@ def _orth_fallback(G: torch.Tensor):
     T = (V / lam.sqrt()[None, :]).float()
     R = (V * lam.sqrt()[None, :]).T.float()
     return T.to(G.device), R.to(G.device)
+
+
+def _transpose_fits(entries: int, n_cols: int, free_bytes: int) -> bool:
+    """Whether ``load`` makes a transposed copy of the matrix.  torch.sort takes up to 2^31 - 1 elements,
+    and the copy, 8 bytes an entry once made, passes through keys, 8-byte positions and their sort
+    buffers: 64 bytes an entry and 24 a column at most, which may take half of what is free."""
+    return entries < 1 << 31 and 64 * entries + 24 * n_cols <= free_bytes // 2
 
 
 class SvdGpu(paralg):
@@ -50,7 +58,8 @@ class SvdGpu(paralg):
         self.paracel_dense_table("AtW", self.N * self.K, handler=update_function)
 
     def load(self, row_ptr: torch.Tensor, cols: torch.Tensor, vals: torch.Tensor):
-        """This rank's rows of A as CSR (int64 row_ptr, int32 global column ids, fp32 values)."""
+        """This rank's rows of A as CSR (int64 row_ptr, int32 global column ids, fp32 values).  Also makes a
+        transposed copy where `_transpose_fits`; larger matrices do without."""
         from ..ops import _lib
         dev = self.device
         self.row_ptr = row_ptr.to(dev, torch.int64).contiguous()
@@ -58,16 +67,27 @@ class SvdGpu(paralg):
         self.vals = vals.to(dev, torch.float32).contiguous()
         _lib.validate_ids(self.cols, 0, self.N, "SVD input (column ids)")
         self.m = self.row_ptr.numel() - 1
+        first, last = (int(self.row_ptr[0].item()), int(self.row_ptr[-1].item())) if self.m > 0 else (0, 0)
+        self.t_ptr = self.t_rows = self.t_vals = None
+        free = torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
+        if not _transpose_fits(last - first, self.N, free):
+            return
         # A^T in the same form: its products then add up in registers.  Scattering an entry at a time
         # into A^T W queues up at the popular columns: 1 ms a product on 6.5 M Zipf(1.1) entries,
         # K = 32, against 0.14 ms for A H.
-        first, last = (int(self.row_ptr[0].item()), int(self.row_ptr[-1].item())) if self.m > 0 else (0, 0)
         c, order = torch.sort(self.cols[first:last], stable=True)
         row_of = torch.repeat_interleave(torch.arange(self.m, device=dev, dtype=torch.int32),
                                          self.row_ptr[1:] - self.row_ptr[:-1])
         self.t_rows, self.t_vals = row_of[order], self.vals[first:last][order]
         self.t_ptr = torch.zeros(self.N + 1, dtype=torch.int64, device=dev)
         self.t_ptr[1:] = torch.cumsum(torch.bincount(c, minlength=self.N), 0)
+
+    def _times_transposed(self, W: torch.Tensor, out: torch.Tensor) -> None:
+        """``out = A^T W`` for this rank's rows."""
+        if self.t_ptr is not None:
+            spmm_csr(self.t_ptr, self.t_rows, self.t_vals, W, out)
+        else:
+            spmm_csr_t(self.row_ptr, self.cols, self.vals, W, out.zero_())
 
     def _reduce(self, key: str, buf: torch.Tensor, cols: int) -> torch.Tensor:
         """Sum over the ranks of what each wrote into ``buf``, the delta buffer of the table ``key``:
@@ -108,7 +128,7 @@ class SvdGpu(paralg):
             W = self._times_inverse(spmm_csr(*A, H), gram(H))
             WtW = self._sum_gram(W)
             buf = self.paracel_delta_buffer("AtW")
-            spmm_csr(self.t_ptr, self.t_rows, self.t_vals, W, buf.view(N, K))
+            self._times_transposed(W, buf.view(N, K))
             AtW = self._reduce("AtW", buf, K)
             H = self._times_inverse(AtW, WtW)
         W = self._times_inverse(spmm_csr(*A, H), gram(H))

@@ -345,3 +345,12 @@ def test_host_rand_refuses_what_the_host_generator_refuses(seed, device, what):
     from paracel_b200.ops.svd import host_rand
     with pytest.raises((ValueError, RuntimeError), match=what):
         host_rand((4,), seed, device)
+
+
+def test_svd_makes_no_transposed_copy_of_what_is_too_large_for_one():
+    """Beyond the sort's element count, or where its buffers take more than half of the free memory."""
+    from paracel_b200.models.svd_gpu import _transpose_fits
+    big = 1 << 40
+    assert _transpose_fits(0, 1, 1 << 20) and _transpose_fits((1 << 31) - 1, 1000, big)
+    assert not _transpose_fits(1 << 31, 1000, big)
+    assert _transpose_fits(1000, 500, 2 * 76_000) and not _transpose_fits(1000, 500, 2 * 76_000 - 1)

@@ -390,3 +390,32 @@ def test_similarity_leaves_out_rows_with_negative_ids():
     assert {r: [c for c, _ in v] for r, v in m.result.items()} == {
         int(ids[r]): [int(ids[c]) for c in order[r]] for r in range(n)}
     m.free()
+
+
+@pytest.mark.parametrize("copy", [True, False])
+def test_svd_of_a_full_rank_matrix_with_and_without_the_transposed_copy(monkeypatch, copy):
+    """Row pointers that do not start at zero, empty rows, against an SVD in 64 bits."""
+    import paracel_b200.models.svd_gpu as sg
+    monkeypatch.setattr(sg, "_transpose_fits", lambda *a: copy)
+    g = torch.Generator(device="cuda").manual_seed(8)
+    n, N, k, lead = 900, 150, 5, 3
+    lens = torch.randint(0, 30, (n,), device="cuda", generator=g)
+    ptr, idx, val = _ragged_csr(n, N, lens, g, lead=lead)
+    A = torch.zeros(n, N, dtype=torch.float64, device="cuda")
+    rows = torch.repeat_interleave(torch.arange(n, device="cuda"), lens)
+    # a strong rank-5 part, so that the iteration has converged after 30 steps
+    U, V = (torch.randn(x, k, dtype=torch.float64, device="cuda", generator=g) for x in (n, N))
+    c = idx[lead:].long()
+    val[lead:] += (8 * (U[rows] * V[c]).sum(1)).float()
+    A.index_put_((rows, c), val[lead:].double(), accumulate=True)
+    m = sg.SvdGpu(N, k, iters=30, device="cuda")
+    m.load(ptr, idx, val)
+    m.solve()
+    assert (m.t_ptr is not None) == copy
+    Ur, S, Vr = torch.linalg.svd(A, full_matrices=False)
+    # Gram matrices in fp32 square the factors' condition: sigma is good to about 2^-24 (s_1 / s_k)^2
+    assert bool(((m.sigma.cuda() - S[:k]).abs() <= 64 * 2.0 ** -24 * float(S[0] / S[k - 1]) ** 2 * S[:k]).all())
+    P = m.U.double() @ torch.diag(m.sigma.cuda()) @ m.V.double().T
+    best = Ur[:, :k] @ torch.diag(S[:k]) @ Vr[:k]
+    assert float((P - best).norm()) <= 1e-3 * float(best.norm())
+    m.free()
