@@ -678,9 +678,9 @@ int launch_warp(const AlsArgs& a, int cls, cudaStream_t stream) {
 
 // k <= 128, n_users < 2^31.  `nnz` is the length of item_idx / rating (user_ptr is ascending within
 // [0, nnz]).  Users with more than `split` ratings are cut into pieces of `piece`.  Workspaces:
-// scratch holds nnz / split slots of K*K + K floats (K = k rounded up to 32 / 64 / 128, 16-byte
-// aligned) and slot_count as many ints; counters 8 ints; seg 3 x seg_cap ints with
-// seg_cap >= n_users + nnz / piece + nnz / split; user_list 4 x n_users ints.  Rows of W of users without
+// scratch holds as many slots of K*K + K floats (K = k rounded up to 32 / 64 / 128, 16-byte aligned) as
+// users are split (nnz / split at most) and slot_count as many ints; counters 8 ints; seg 3 x seg_cap ints
+// with seg_cap >= n_users + nnz / piece + slots; user_list 4 x n_users ints.  Rows of W of users without
 // ratings are not written.
 PCL_API int pcl_als_solve(const long long* user_ptr, const int* item_idx, const float* rating, const float* H,
                           float* W, float* scratch, int* slot_count, int* counters, int* seg, int* user_list,

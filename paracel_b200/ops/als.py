@@ -31,12 +31,15 @@ def als_solve(user_ptr: torch.Tensor, item_idx: torch.Tensor, rating: torch.Tens
     nnz = item_idx.numel()
     if n_users <= 0 or nnz == 0:
         return W
-    # At most 2048 users are split, which bounds the scratch (135 MB at rank 128) without asking the
-    # device how many there are; a split user's pieces are a quarter as long, so that the last ones
-    # to run are short.
-    split = max(int(seg_len), (nnz + 2047) // 2048)
+    # No accumulator takes more than seg_len ratings in a row: its rounding errors grow with that.  A
+    # split user's pieces are a quarter as long, so that the last ones to run are short.
+    split = max(int(seg_len), 1)
     piece = max(split // 4, 256)
+    # One scratch slot per split user.  nnz / split bounds them without asking the device (as long as
+    # that is 4096 at most, 270 MB at rank 128), a read of the true number costs some 50 us.
     slots = nnz // split + 1
+    if slots > 4096:
+        slots = int(((user_ptr[1:] - user_ptr[:-1]) > split).sum().item()) + 1
     seg_cap = n_users + nnz // piece + slots
     scratch = torch.empty(slots * (K * K + K), device=dev)
     ints = torch.empty(slots + 8 + 3 * seg_cap + 4 * n_users, dtype=torch.int32, device=dev)

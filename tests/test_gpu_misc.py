@@ -419,3 +419,15 @@ def test_svd_of_a_full_rank_matrix_with_and_without_the_transposed_copy(monkeypa
     best = Ur[:, :k] @ torch.diag(S[:k]) @ Vr[:k]
     assert float((P - best).norm()) <= 1e-3 * float(best.norm())
     m.free()
+
+
+def test_als_accumulators_take_no_more_than_seg_len_ratings_in_a_row():
+    """2050 users of 16,300 equal ratings: one fp32 chain over a user's ratings is off by 1.9e-4, chains of
+    4096 by at most half a unit of the sum per term, 4096 * 2^-25."""
+    from paracel_b200.ops.als import als_solve
+    users, n = 2050, 16_300
+    r = 1 + 2.0 ** -11 - 2.0 ** -14
+    ptr = torch.arange(users + 1, device="cuda") * n
+    idx = torch.zeros(users * n, dtype=torch.int32, device="cuda")
+    W = als_solve(ptr, idx, torch.full((users * n,), r, device="cuda"), torch.ones(1, 1, device="cuda"), lam=1.0)
+    assert float((W.double() / (n * r / (n + 1)) - 1).abs().max()) <= (4096 + 8) * 2.0 ** -25
