@@ -229,6 +229,7 @@ constexpr float SG_FX = 16384.f, SG_FXI = 1.f / 16384.f;
 #define SG_ROWS_N 4
 #endif
 constexpr int SG_ROWS = SG_ROWS_N;
+constexpr int SG_LONG = 4;
 
 // residual of one row from its margin z; adds the row's loss
 __device__ __forceinline__ float sg_residual(const SparseGradArgs& a, float z, float yy, double& loss) {
@@ -257,12 +258,15 @@ __device__ __forceinline__ void sg_scatter(const SparseGradArgs& a, int* s_hot, 
 // pointers, column ids, gather of theta, then the atomics), and with one row per warp the SM had
 // only as many chains in flight as resident warps (long scoreboard 17 stall cycles per issue).
 // Rows of up to 64 non-zeros keep their ids and values in registers between the margin and the
-// scatter; longer rows take the loop form.
+// scatter.  If a step has a longer row, its rows are taken one after the other, 32 SG_LONG entries in
+// flight at a time (rows of up to that many keep them in registers too).
 // Measured on 50 M x 2^24 with 40 non-zeros per row: 1 / 2 / 4 / 8 rows per step gave 2.04 / 3.16 /
-// 3.36 / 2.06 G samples/s (eight rows cost too many registers).  The stream (limits, ids, values) is read
-// one step ahead and past the caches' stock of weights: an epoch over 8 M such rows, four
-// minibatches, 2483 -> 2121 us; 2 M rows of 20 values 527 -> 399 us.  Three CTAs per SM without the few
-// spilled registers, or two rows per step with five CTAs, gave 2280 us.
+// 3.36 / 2.06 G samples/s (eight rows cost too many registers).  The stream (limits, ids, values) of short
+// rows is read one step ahead and past the caches' stock of weights: 2 M such rows 540 -> 412 us, with
+// values 561 -> 426 us, against all of it read in its own step.
+// Long rows as a loop over 32 entries, and their steps' registers filled for nothing: 2 M rows of 80 entries
+// 1350 us, 1 M of 90 with values 620 us; SG_LONG 2 / 3 / 4 / 6: 1061 / 817 / 832 / 866 and 498 / 371 / 385 /
+// 412 us, rows of 300 entries 354 / 311 / 291 / 307 us.
 template <bool VALS, bool FX>
 __global__ void __launch_bounds__(256, 4) sparse_grad_kernel(SparseGradArgs a) {
   extern __shared__ int s_hot[];
@@ -271,9 +275,9 @@ __global__ void __launch_bounds__(256, 4) sparse_grad_kernel(SparseGradArgs a) {
   __syncthreads();
   double loss = 0.0;
   const long long stride = (long long)gridDim.x * wpb;
-  // limits of a step's rows and ids and values of short rows, read one step ahead
-  long long rb[SG_ROWS];
-  int len[SG_ROWS], c[2 * SG_ROWS];
+  // limits of a step's rows and, if all of them are short, their ids and values, read one step ahead
+  bool shortrows = true;
+  int c[2 * SG_ROWS];
   float v[VALS ? 2 * SG_ROWS : 1];
   long long nb[SG_ROWS], ne[SG_ROWS];
   auto limits = [&](long long row0) {
@@ -286,17 +290,15 @@ __global__ void __launch_bounds__(256, 4) sparse_grad_kernel(SparseGradArgs a) {
     }
   };
   auto entries = [&]() {
+    shortrows = true;
 #pragma unroll
-    for (int k = 0; k < SG_ROWS; ++k) {
-      rb[k] = nb[k];
-      len[k] = (int)(ne[k] - nb[k]);
-    }
+    for (int k = 0; k < SG_ROWS; ++k) shortrows &= ne[k] - nb[k] <= 64;
 #pragma unroll
     for (int q = 0; q < 2 * SG_ROWS; ++q) {
-      const int i = (q & 1) * 32 + lane;
-      const bool in = i < len[q >> 1];
-      c[q] = in ? __ldcs(a.cols + rb[q >> 1] + i) : -1;
-      if (VALS) v[VALS ? q : 0] = in ? __ldcs(a.vals + rb[q >> 1] + i) : 1.f;
+      const long long p = nb[q >> 1] + (q & 1) * 32 + lane;
+      const bool in = shortrows && p < ne[q >> 1];
+      c[q] = in ? __ldcs(a.cols + p) : -1;
+      if (VALS) v[VALS ? q : 0] = in ? __ldcs(a.vals + p) : 1.f;
     }
   };
   long long row0 = (long long)blockIdx.x * wpb + warp;
@@ -306,11 +308,8 @@ __global__ void __launch_bounds__(256, 4) sparse_grad_kernel(SparseGradArgs a) {
   }
   for (; row0 < a.n; row0 += SG_ROWS * stride) {
     const long long next = row0 + SG_ROWS * stride;
-    limits(next);                                // rows past the end: empty
-    bool shortrows = true;
-#pragma unroll
-    for (int k = 0; k < SG_ROWS; ++k) shortrows &= len[k] <= 64;
     if (shortrows) {
+      limits(next);                              // rows past the end: empty
       float t[2 * SG_ROWS];
 #pragma unroll
       for (int q = 0; q < 2 * SG_ROWS; ++q) t[q] = c[q] >= 0 ? __ldg(a.theta + c[q]) : 0.f;
@@ -342,21 +341,51 @@ __global__ void __launch_bounds__(256, 4) sparse_grad_kernel(SparseGradArgs a) {
       }
       continue;
     }
+    // some row is long: lanes 2 k and 2 k + 1 hold the limits of row k of this step and of the next, which
+    // leaves the registers to the loops
+    auto lane_limit = [&](long long first) -> long long {
+      const long long row = first + (lane >> 1) * stride;
+      return lane < 2 * SG_ROWS && row < a.n ? __ldg(a.row_ptr + row + (lane & 1)) : 0;
+    };
+    const long long lim = lane_limit(row0), ahead = lane_limit(next);
+#pragma unroll 1
     for (int k = 0; k < SG_ROWS; ++k) {
       const long long row = row0 + k * stride;
       if (row >= a.n) break;
-      const long long b = rb[k], e = b + len[k];
+      const long long b = __shfl_sync(0xffffffffu, lim, 2 * k), e = __shfl_sync(0xffffffffu, lim, 2 * k + 1);
+      const float y1 = __ldg(a.y + row);
+      int cl[SG_LONG];
+      float vl[SG_LONG];
+      auto fetch = [&](long long q) {              // the row's entries q .. q + 32 SG_LONG - 1, all loads in flight
+#pragma unroll
+        for (int j = 0; j < SG_LONG; ++j) {
+          const long long p = q + 32 * j + lane;
+          cl[j] = p < e ? __ldg(a.cols + p) : -1;
+          vl[j] = VALS && p < e ? __ldg(a.vals + p) : 1.f;
+        }
+      };
       float zz = 0.f;
-      for (long long q = b + lane; q < e; q += 32) {
-        const float vv = VALS ? a.vals[q] : 1.f;
-        zz = fmaf(vv, __ldg(a.theta + a.cols[q]), zz);
+#pragma unroll 1
+      for (long long q = b; q < e; q += 32 * SG_LONG) {
+        fetch(q);
+#pragma unroll
+        for (int j = 0; j < SG_LONG; ++j)
+          if (cl[j] >= 0) zz = fmaf(vl[j], __ldg(a.theta + cl[j]), zz);
       }
       zz = pcl_warp_sum(zz);
-      const float r = sg_residual(a, zz, a.y[row], loss);
-      for (long long q = b + lane; q < e; q += 32) {
-        const float vv = VALS ? a.vals[q] : 1.f;
-        sg_scatter<FX>(a, s_hot, a.cols[q], r * vv);
+      const float r = sg_residual(a, zz, y1, loss);
+#pragma unroll 1
+      for (long long q = b; q < e; q += 32 * SG_LONG) {
+        if (e - b > 32 * SG_LONG) fetch(q);        // else they are still there
+#pragma unroll
+        for (int j = 0; j < SG_LONG; ++j)
+          if (cl[j] >= 0) sg_scatter<FX>(a, s_hot, cl[j], r * vl[j]);
       }
+    }
+#pragma unroll
+    for (int k = 0; k < SG_ROWS; ++k) {
+      nb[k] = __shfl_sync(0xffffffffu, ahead, 2 * k);
+      ne[k] = __shfl_sync(0xffffffffu, ahead, 2 * k + 1);
     }
     entries();
   }

@@ -431,3 +431,36 @@ def test_als_accumulators_take_no_more_than_seg_len_ratings_in_a_row():
     idx = torch.zeros(users * n, dtype=torch.int32, device="cuda")
     W = als_solve(ptr, idx, torch.full((users * n,), r, device="cuda"), torch.ones(1, 1, device="cuda"), lam=1.0)
     assert float((W.double() / (n * r / (n + 1)) - 1).abs().max()) <= (4096 + 8) * 2.0 ** -25
+
+
+@pytest.mark.parametrize("valued", [True, False])
+@pytest.mark.parametrize("logistic", [True, False])
+def test_sparse_gradient_of_long_rows(logistic, valued):
+    """Rows around the 64 entries of the short form and the 128 a long row keeps in registers, mixed and alone."""
+    from paracel_b200.ops.linear import sparse_grad
+    g = torch.Generator(device="cuda").manual_seed(9)
+    F = 12_000
+    for pick in ([63, 64, 65], [127, 128, 129, 1], [65], [400, 0, 128, 256]):
+        n = 3001
+        lens = torch.tensor(pick, device="cuda")[torch.randint(0, len(pick), (n,), device="cuda", generator=g)]
+        ptr = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+        ptr[1:] = lens.cumsum(0)
+        cols = (torch.rand(int(ptr[-1]), device="cuda", generator=g) ** 3 * F).int().clamp(max=F - 1)
+        vals = torch.rand(cols.numel(), device="cuda", generator=g) if valued else None
+        v64 = vals.double() if valued else torch.ones(cols.numel(), device="cuda").double()
+        theta = 0.05 * torch.randn(F, device="cuda", generator=g)
+        y = (torch.rand(n, device="cuda", generator=g) < 0.5).float()
+        row = torch.repeat_interleave(torch.arange(n, device="cuda"), lens)
+        zero = torch.zeros(n, dtype=torch.float64, device="cuda")
+        z = zero.index_add(0, row, v64 * theta.double()[cols.long()])
+        zmag = zero.index_add(0, row, v64 * theta.double()[cols.long()].abs())
+        r = y.double() - (torch.sigmoid(z) if logistic else z)
+        fzero = torch.zeros(F, dtype=torch.float64, device="cuda")
+        ref = fzero.index_add(0, cols.long(), r[row] * v64)
+        mag = fzero.index_add(0, cols.long(), v64 * (1 + zmag[row]))
+        cnt = torch.bincount(cols.long(), minlength=F).double()
+        grad, loss = torch.zeros(F, device="cuda"), torch.zeros(1, dtype=torch.float64, device="cuda")
+        sparse_grad(ptr, cols, vals, y, theta, grad, loss, logistic=logistic)
+        # half a unit of the fixed-point table per term; margins of up to 400 terms; fp32 sums of cnt terms
+        bound = (cnt * 2.0 ** -15 if logistic else 0) + (cnt + 420) * 2.0 ** -23 * mag
+        assert bool(((grad.double() - ref).abs() <= bound + 1e-30).all()), pick
