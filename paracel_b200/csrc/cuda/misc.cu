@@ -129,6 +129,16 @@ inline int km_few_warps(long long copy_bytes, int groups_per_warp) {
   return w * groups_per_warp >= 5 ? w : 0;
 }
 
+// Clearing and adding up a block's own sums takes a time that grows with k, and more with wide rows,
+// whose sums leave room for fewer warps; the reductions queue up for n / k of them per address.  The line
+// fits both sides measured at 10 k, 100 k and 900 k points of 4 to 512 columns in 2 to 200 clusters: 10 k x 8 in 30
+// clusters 14.4 us with reductions against 10.3 here, in 64 12.3 against 14.3, in 200 11 against 32;
+// 100 k x 64 in 64 83 against 37, in 100 52 against 56; 100 k x 16 in 120 43 against 29, in 200 32 against 47.
+inline bool km_few_pays(long long n, int d, int k) {
+  const long long w = d > 128 || d < 68 ? 20 + d : 88;
+  return k < 1 << 16 && (long long)k * k * w <= 8 * n;
+}
+
 template <int LG, int PIECES>
 int launch_km_few(const float* X, const int* assign, long long n, int d, int k, float* sums, float* counts,
                   bool* taken, cudaStream_t stream) {
@@ -410,7 +420,7 @@ PCL_API int pcl_kmeans_accumulate(const float* X, const int* assign, long long n
   long long blocks = (n + 7) / 8;
   if (blocks > 148 * 8) blocks = 148 * 8;
   const bool vec = (d % 4 == 0) && d <= 512 && (((uintptr_t)X | (uintptr_t)sums) & 15) == 0;
-  if (vec && k > 0) {
+  if (vec && k > 0 && km_few_pays(n, d, k)) {
     bool taken = false;
     int rc;
     if (d <= 4) rc = launch_km_few<1, 1>(X, assign, n, d, k, sums, counts, &taken, stream);

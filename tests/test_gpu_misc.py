@@ -433,6 +433,23 @@ def test_als_accumulators_take_no_more_than_seg_len_ratings_in_a_row():
     assert float((W.double() / (n * r / (n + 1)) - 1).abs().max()) <= (4096 + 8) * 2.0 ** -25
 
 
+@pytest.mark.parametrize("d,k,n", [(4, 20, 1200), (16, 40, 7200), (32, 64, 26624), (64, 30, 9450), (100, 30, 9900),
+                                   (128, 20, 4400), (256, 12, 4968), (512, 6, 2394)])
+def test_kmeans_accumulate_on_both_sides_of_the_point_count_that_picks_its_sums(d, k, n):
+    from paracel_b200.ops.misc import kmeans_accumulate
+    g = torch.Generator(device="cuda").manual_seed(d + k)
+    for m in (n - 1, n):
+        X = torch.randn(m, d, device="cuda", generator=g)
+        a = torch.randint(0, k, (m,), device="cuda", generator=g, dtype=torch.int32)
+        sums, counts = torch.zeros(k, d, device="cuda"), torch.zeros(k, device="cuda")
+        kmeans_accumulate(X, a, sums, counts)
+        ref = torch.zeros(k, d, dtype=torch.float64, device="cuda").index_add_(0, a.long(), X.double())
+        mag = torch.zeros(k, d, dtype=torch.float64, device="cuda").index_add_(0, a.long(), X.double().abs())
+        cnt = torch.bincount(a.long(), minlength=k).double()
+        assert torch.equal(counts.double(), cnt)
+        assert bool(((sums.double() - ref).abs() <= (cnt[:, None] + 1) * 2.0 ** -24 * mag).all())
+
+
 @pytest.mark.parametrize("valued", [True, False])
 @pytest.mark.parametrize("logistic", [True, False])
 def test_sparse_gradient_of_long_rows(logistic, valued):
