@@ -263,8 +263,9 @@ __global__ void __launch_bounds__(256) topk_rows_kernel(const float* S, long lon
 // packed multiply-add; with fewer than ten blocks several warps share one and split the rows.  A row
 // costs a warp three 16-byte shared-memory loads (12 passes) for 1024 multiply-adds; with 2 x 2
 // values per thread of one 16 x 16 grid it took 32 passes (mean of 400 k x 32 and 100 k x 32: 52 -> 36 us).
-// Rows arrive by asynchronous copies one stage ahead.
-constexpr int GM_T = 320, GM_RS = 40;
+// Rows arrive by asynchronous copies one stage ahead.  The registers' sums go to shared memory after
+// GM_RUN rows: rounding errors grow with the length of a chain of additions.
+constexpr int GM_T = 320, GM_RS = 40, GM_RUN = 1280;
 
 template <int KB>
 __global__ void __launch_bounds__(GM_T) gram_kernel(const float* H, long long n, int k, int vec, float* out) {
@@ -312,7 +313,31 @@ __global__ void __launch_bounds__(GM_T) gram_kernel(const float* H, long long n,
     }
     __pipeline_commit();
   };
-  int buf = 0;
+  float* sS = sm + 2 * GM_RS * K;
+  bool fresh = true;
+  auto add_up = [&]() {                            // the registers' sums into shared memory, one group after the other
+#pragma unroll 1
+    for (int g = 0; g < GR; ++g) {
+      if (has_blk && grp == g) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            float v[2];
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(v[0]), "=f"(v[1]) : "l"(acc[i][j]));
+            acc[i][j] = 0ull;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              float* p = sS + (row0 + i) * K + col0 + 16 * (j >> 1) + 2 * (j & 1) + q;
+              *p = fresh && g == 0 ? v[q] : *p + v[q];
+            }
+          }
+      }
+      __syncthreads();
+    }
+    fresh = false;
+  };
+  int buf = 0, since = 0;
   stage(blockIdx.x, 0);
   for (long long s = blockIdx.x; s < stages; s += gridDim.x, buf ^= 1) {
     stage(s + gridDim.x, buf ^ 1);
@@ -336,27 +361,13 @@ __global__ void __launch_bounds__(GM_T) gram_kernel(const float* H, long long n,
       }
     }
     __syncthreads();
+    if (++since == GM_RUN * GR / GM_RS) {
+      since = 0;
+      add_up();
+    }
   }
   __pipeline_wait_prior(0);
-  float* sS = sm + 2 * GM_RS * K;
-#pragma unroll 1
-  for (int g = 0; g < GR; ++g) {
-    if (has_blk && grp == g) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float v[2];
-          asm("mov.b64 {%0, %1}, %2;" : "=f"(v[0]), "=f"(v[1]) : "l"(acc[i][j]));
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            float* p = sS + (row0 + i) * K + col0 + 16 * (j >> 1) + 2 * (j & 1) + q;
-            *p = g == 0 ? v[q] : *p + v[q];
-          }
-        }
-    }
-    __syncthreads();
-  }
+  add_up();
   for (int e = tid; e < k * k; e += GM_T) {
     const int r = e / k, c = e % k;
     const float v = c <= r ? sS[r * K + c] : sS[c * K + r];
@@ -369,7 +380,7 @@ int launch_gram(const float* H, long long n, int k, float* out, cudaStream_t str
   const size_t smem = (2 * (size_t)GM_RS * 16 * KB + 256 * (size_t)KB * KB) * sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(gram_kernel<KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  const long long need = (n + GM_RS - 1) / GM_RS;
+  const long long need = (n + 63) / 64;            // every block's sums are one more addition per entry
   const int blocks = need < 148 * 2 ? (int)need : 148 * 2;
   const int vec = (k & 3) == 0 && (reinterpret_cast<uintptr_t>(H) & 15) == 0;
   gram_kernel<KB><<<blocks, GM_T, smem, stream>>>(H, n, k, vec, out);
