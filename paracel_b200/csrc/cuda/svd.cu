@@ -16,13 +16,18 @@
 namespace {
 
 // Work is cut by entries, not by rows: a group of G lanes (the smallest power of two with 16 bytes
-// of a K-wide row per lane) owns SP_L consecutive entries whatever rows they belong to, so a row with a
+// of a K-wide row per lane) owns L consecutive entries whatever rows they belong to, so a row with a
 // million entries is spread over the chip and a row with two costs two.  (A warp per row took 13.7 ms
 // on 400 k rows x 16 M Zipf(1.1) entries, K = 32, of which one warp's chain over the hottest row was all
-// but half a millisecond, and used 8 of its 32 lanes; SPMM_MEAS.)  What is left is bound by the
+// but half a millisecond, and used 8 of its 32 lanes.)  What is left is bound by the
 // gathers of 4 K bytes per entry out of L2: four are in flight per group before the first is used.
+// Rows of even length, against a warp per row: 500 k x 40 entries out of 20 k columns, K = 16 / 32 / 52 / 128,
+// 157 / 267 / 424 / 679 us against 672 / 674 / 676 / 691; 400 k x 16 out of 100 k 69 / 101 / 151 / 282 against
+// 243 / 245 / 246 / 258.  Short rows with K > 64 and small matrices stay behind it (400 k x 5, K = 128, 150 us
+// against 128; 20 k x 15, K = 128, 27.6 against 20.6): more row ends per entry, and a chain of searches before
+// the first gather.
 // A segment that holds a whole row stores it; the pieces of a cut row are added with vector
-// reductions into `out`, which the launcher clears.
+// reductions into `out`, cleared before by spmm_clear_kernel.
 // TRANS: out[c, :] += v * W[r, :] instead (a reduction per entry; W's row stays in registers).
 constexpr int SP_ROWS = 1024;   // row ends of a block kept in shared memory up to this many rows
 
@@ -44,7 +49,7 @@ __device__ __forceinline__ long long row_of_entry(const long long* row_ptr, long
 }
 
 template <int G, bool TRANS>
-__global__ void __launch_bounds__(256) spmm_kernel(const long long* __restrict__ row_ptr,
+__global__ void __launch_bounds__(256, G >= 16 && !TRANS ? 5 : 0) spmm_kernel(const long long* __restrict__ row_ptr,
                                                    const int* __restrict__ cols,
                                                    const float* __restrict__ vals, long long n_rows,
                                                    long long n_ent, int L, const float* __restrict__ X,
@@ -129,6 +134,19 @@ __global__ void __launch_bounds__(256) spmm_kernel(const long long* __restrict__
     }
     float4 h[U];
     if constexpr (!TRANS) {
+      // all of the current row: without the questions below 889 -> 693 us on 100 k x 200 entries, K = 128; with
+      // narrow groups a warp would go both ways (400 k x 5, K = 32: 77 -> 83 us)
+      if (G >= 16 && p0 >= gs && p0 + U <= (end < ge ? end : ge)) {
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+          h[j] = on ? __ldg(reinterpret_cast<const float4*>(X + (long long)c[j] * K + 4 * gl)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+          acc.x = fmaf(v[j], h[j].x, acc.x); acc.y = fmaf(v[j], h[j].y, acc.y);
+          acc.z = fmaf(v[j], h[j].z, acc.z); acc.w = fmaf(v[j], h[j].w, acc.w);
+        }
+        continue;
+      }
 #pragma unroll
       for (int j = 0; j < U; ++j)
         h[j] = (on && p0 + j >= gs && p0 + j < ge) ? __ldg(reinterpret_cast<const float4*>(X + (long long)c[j] * K + 4 * gl))
@@ -158,17 +176,48 @@ __global__ void __launch_bounds__(256) spmm_kernel(const long long* __restrict__
   if constexpr (!TRANS) flush(cut || end > ge);
 }
 
+// Zeros in the rows of `out` that spmm_kernel adds to (their entries lie in several segments of L) or
+// does not touch (no entries).  Clearing all of `out` wrote it twice: 400 k rows x 5 entries, K = 128,
+// 177 us, with this kernel 152.
+__global__ void __launch_bounds__(256) spmm_clear_kernel(const long long* __restrict__ row_ptr, long long n_rows,
+                                                         long long n_ent, int L, int K, float* __restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  const long long r0 = ((long long)blockIdx.x * 256 + threadIdx.x) / 32 * 32, r = r0 + lane;
+  bool zero = false;
+  if (r < n_rows) {
+    const long long b = __ldg(row_ptr + r), e = __ldg(row_ptr + r + 1);
+    zero = e <= b || e > n_ent || ((b ^ (e - 1)) & ~(long long)(L - 1)) != 0;   // L is a power of two
+  }
+  for (unsigned todo = __ballot_sync(0xffffffffu, zero); todo; todo &= todo - 1) {
+    float* o = out + (r0 + __ffs(todo) - 1) * K + 4 * lane;
+    if (4 * lane < K) *reinterpret_cast<float4*>(o) = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+
 template <bool TRANS>
 int launch_spmm(const long long* row_ptr, const int* cols, const float* vals, long long n_rows,
                 long long n_ent, const float* X, int K, float* out, cudaStream_t stream) {
   int G = 1;
   while (4 * G < K) G *= 2;
-  // entries per group: 128, fewer while the chip's groups (2048 threads on each of 148 SMs) would
-  // not all get a segment
-  int L = 128;
-  while (L > 16 && n_ent / L < 148LL * 2048 / G) L /= 2;
+  // Entries per group.  Narrow groups: 128, fewer while the chip's groups (2048 threads on each of 148 SMs)
+  // would not all get a segment.  From K = 36 on four times as many if that leaves four segments each (fewer
+  // row searches: 20 M entries, K = 128, 724 us at 128 and 679 at 512), and fewer only for a third of
+  // the groups (300 k entries, K = 128: 27.6 us against 33.8).
+  const bool wide = G >= 16 && !TRANS;
+  int L = wide ? 512 : 128;
+  while (L > 128 && n_ent / L < 4 * 148LL * 2048 / G) L /= 2;
+  while (L > 16 && n_ent / L < 148LL * (wide ? 640 : 2048) / G) L /= 2;
   const long long blocks = (n_ent + (256 / G) * (long long)L - 1) / ((256 / G) * (long long)L);
-  if (blocks > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
+  const long long clear = (n_rows + 255) / 256;
+  if (blocks > 0x7fffffffLL || clear > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
+  if constexpr (!TRANS) {
+    if (n_rows * K <= 1 << 20) {                   // up to 4 MB clearing all is 2 us faster
+      const cudaError_t e = cudaMemsetAsync(out, 0, (size_t)n_rows * K * sizeof(float), stream);
+      if (e != cudaSuccess) return (int)e;
+    } else {
+      spmm_clear_kernel<<<(int)clear, 256, 0, stream>>>(row_ptr, n_rows, n_ent, L, K, out);
+    }
+  }
 #define PCL_SPMM(GG)                                                                                     \
   case GG:                                                                                               \
     spmm_kernel<GG, TRANS><<<(int)blocks, 256, 0, stream>>>(row_ptr, cols, vals, n_rows, n_ent, L, X, K, out); \
@@ -415,9 +464,7 @@ PCL_API int pcl_spmm_csr(const long long* row_ptr, const int* cols, const float*
                          long long n_ent, const float* H, int K, float* out, cudaStream_t stream) {
   if (n_rows <= 0) return 0;
   if (K <= 0 || K > 128 || (K & 3)) return (int)cudaErrorInvalidValue;
-  cudaError_t e = cudaMemsetAsync(out, 0, (size_t)n_rows * K * sizeof(float), stream);
-  if (e != cudaSuccess) return (int)e;
-  if (n_ent <= 0) return 0;
+  if (n_ent <= 0) return (int)cudaMemsetAsync(out, 0, (size_t)n_rows * K * sizeof(float), stream);
   return launch_spmm<false>(row_ptr, cols, vals, n_rows, n_ent, H, K, out, stream);
 }
 

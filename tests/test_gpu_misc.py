@@ -461,6 +461,26 @@ def test_gram_chains_are_bounded(k):
     assert float((G.double() / (n * h * h) - 1).abs().max()) <= chain * 2.0 ** -25
 
 
+@pytest.mark.parametrize("n,per,K", [(9001, 130, 128), (40_003, 7, 32), (30_001, 16, 52), (120_001, 200, 128)])
+def test_csr_product_writes_every_row_of_a_dirty_output(n, per, K):
+    """Outputs beyond 4 MB are cleared by rows: those without entries and those cut by a segment's end
+    (of 512 entries in the last case), while the others are stored once."""
+    from paracel_b200.ops.svd import spmm_csr
+    g = torch.Generator(device="cuda").manual_seed(n)
+    lens = torch.full((n,), per, device="cuda")
+    lens[::11] = 0
+    lens[5], lens[-1] = 3000, 0
+    ptr, idx, val = _ragged_csr(n, 701, lens, g)
+    H = torch.randn(701, K, device="cuda", generator=g)
+    out = torch.full((n, K), float("nan"), device="cuda")
+    spmm_csr(ptr, idx, val, H, out)
+    assert bool(torch.isfinite(out).all()) and not bool(out[::11].any())
+    for r in [1, 4, 5, 6, n // 2, n - 3] + list(range(2000, 2060)):
+        a, b = int(ptr[r]), int(ptr[r + 1])
+        prod = val[a:b].double()[:, None] * H[idx[a:b].long()].double()
+        assert bool(((out[r].double() - prod.sum(0)).abs() <= (b - a + 2) * 2.0 ** -24 * prod.abs().sum(0)).all())
+
+
 @pytest.mark.parametrize("valued", [True, False])
 @pytest.mark.parametrize("logistic", [True, False])
 def test_sparse_gradient_of_long_rows(logistic, valued):
