@@ -26,11 +26,19 @@ from ..ops.svd import chol_factor, host_rand, rows_times, spmm_csr, spmm_csr_t
 from ..paralg import paralg
 
 
+# Pivots and eigenvalues of a Gram matrix summed in fp32 are rounding noise below about this much of the
+# largest, and a direction scaled by one over its noise spoils the others.  With cuts of 1e-10 and 1e-12 a
+# singular value of an exact rank-12 matrix was off by more than 0.2 % in one solve of eight and those of a
+# rank-60 one by a factor; cuts from 2^-25 to 2^-22 are good to 1e-6 on both.  Larger ones lose
+# singular values of a thousandth of the largest.
+_GRAM_NOISE = 2.0 ** -24
+
+
 def _orth_fallback(G: torch.Tensor):
     """(T, R) from the eigen-decomposition of a semi-definite Gram matrix restricted to its
     numerical range: Q = M T is orthonormal and M = Q R."""
     lam, V = torch.linalg.eigh(G.double().cpu())
-    keep = lam > 1e-12 * lam.max()
+    keep = lam > _GRAM_NOISE * lam.max()
     lam, V = lam[keep], V[:, keep]
     T = (V / lam.sqrt()[None, :]).float()
     R = (V * lam.sqrt()[None, :]).T.float()
@@ -108,14 +116,14 @@ class SvdGpu(paralg):
         the pseudo-inverse when G is rank deficient (the oversampled factors can be)."""
         if M.shape[0] == 0:
             return M
-        T, _, info = chol_factor(G)
+        T, _, info = chol_factor(G, rel_tol=_GRAM_NOISE)
         if info != 0:
             Tf, _ = _orth_fallback(G)
             return (M @ Tf) @ Tf.T
         return rows_times(M, T, twice=True)
 
     def _orth(self, G: torch.Tensor):
-        T, R, info = chol_factor(G, rel_tol=1e-7)
+        T, R, info = chol_factor(G, rel_tol=_GRAM_NOISE)
         if info != 0:
             return _orth_fallback(G)
         return T, R

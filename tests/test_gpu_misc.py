@@ -512,3 +512,30 @@ def test_sparse_gradient_of_long_rows(logistic, valued):
         # half a unit of the fixed-point table per term; margins of up to 400 terms; fp32 sums of cnt terms
         bound = (cnt * 2.0 ** -15 if logistic else 0) + (cnt + 420) * 2.0 ** -23 * mag
         assert bool(((grad.double() - ref).abs() <= bound + 1e-30).all()), pick
+
+
+@pytest.mark.parametrize("spectrum", ["rank 3", "rank 12", "full"])
+def test_svd_of_rank_deficient_and_ill_conditioned_matrices(spectrum):
+    """Directions of a Gram matrix below its fp32 rounding are noise and must not be inverted.  What is kept
+    is good to K 2^-24 (s_1 / s_k)^2, the rounding of the largest eigenvalue against the smallest."""
+    from paracel_b200.models.svd_gpu import SvdGpu
+    m, n = 80, 30
+    for seed in range(8):
+        g = torch.Generator().manual_seed(seed)
+        if spectrum == "full":
+            k = 8
+            U = torch.linalg.qr(torch.randn(m, n, dtype=torch.float64, generator=g)).Q
+            V = torch.linalg.qr(torch.randn(n, n, dtype=torch.float64, generator=g)).Q
+            s = torch.cat([torch.logspace(0, -2, k, dtype=torch.float64),
+                           0.003 * 0.8 ** torch.arange(n - k, dtype=torch.float64)])
+            M = (U * s) @ V.T
+        else:
+            k = int(spectrum.split()[1])
+            M = torch.randn(m, k, dtype=torch.float64, generator=g) @ torch.randn(k, n, dtype=torch.float64, generator=g)
+        ref = torch.linalg.svdvals(M)[:k]
+        sv = SvdGpu(n, k, device="cuda", seed=seed)
+        sv.load(torch.arange(0, m * n + 1, n), torch.arange(n).repeat(m).int(), M.reshape(-1).float())
+        sv.solve()
+        assert sv.sigma.numel() == k
+        assert bool(((sv.sigma - ref).abs() <= sv.K * 2.0 ** -24 * float(ref[0] / ref[-1]) ** 2 * ref).all()), seed
+        sv.free()
