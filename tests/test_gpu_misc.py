@@ -539,3 +539,21 @@ def test_svd_of_rank_deficient_and_ill_conditioned_matrices(spectrum):
         assert sv.sigma.numel() == k
         assert bool(((sv.sigma - ref).abs() <= sv.K * 2.0 ** -24 * float(ref[0] / ref[-1]) ** 2 * ref).all()), seed
         sv.free()
+
+
+@pytest.mark.parametrize("width", [8, 64, 100, 252])
+def test_narrow_int_rows_pull_push_match_torch(width):
+    """Rows pushed int by int (below 128) and in pieces; pulled one piece per lane up to 128 ints."""
+    from paracel_b200.ps.tables import RowTable
+    g = torch.Generator(device="cuda").manual_seed(width)
+    t = RowTable(500, width, dtype=torch.int32, device="cuda:0")
+    t.shard.copy_(torch.randint(-9, 9, (500, width), device="cuda", generator=g))
+    before, ids = t.shard.clone(), torch.randperm(500, device="cuda", generator=g)[:333]
+    cur, old = (torch.zeros(333, width, dtype=torch.int32, device="cuda") for _ in range(2))
+    t.pull(ids, cur, old)
+    assert torch.equal(cur, before[ids]) and torch.equal(old, cur)
+    new = cur + torch.randint(-2, 3, cur.shape, device="cuda", generator=g, dtype=torch.int32)
+    t.push(ids, new, old)
+    before[ids] = new
+    assert torch.equal(t.shard, before) and torch.equal(old, new)
+    t.free()
