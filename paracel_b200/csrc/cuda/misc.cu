@@ -270,7 +270,7 @@ constexpr int GM_T = 320, GM_RS = 40, GM_RUN = 1280;
 template <int KB>
 __global__ void __launch_bounds__(GM_T) gram_kernel(const float* H, long long n, int k, int vec, float* out) {
   constexpr int K = 16 * KB, B = KB / 2, NB = B * (B + 1) / 2, GR = 10 / NB;
-  extern __shared__ __align__(16) float sm[];      // two stages of GM_RS x K rows, then the K x K sums
+  extern __shared__ __align__(16) float sm[];      // two stages of GM_RS x K rows, then the groups' K x K sums
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int blk = warp % NB, grp = warp / NB;
   const bool has_blk = grp < GR;
@@ -313,27 +313,23 @@ __global__ void __launch_bounds__(GM_T) gram_kernel(const float* H, long long n,
     }
     __pipeline_commit();
   };
-  float* sS = sm + 2 * GM_RS * K;
+  float* sS = sm + 2 * GM_RS * K + (has_blk ? grp : 0) * K * K;   // sums of this warp's group
   bool fresh = true;
-  auto add_up = [&]() {                            // the registers' sums into shared memory, one group after the other
-#pragma unroll 1
-    for (int g = 0; g < GR; ++g) {
-      if (has_blk && grp == g) {
+  auto add_up = [&]() {                            // the registers' sums into shared memory
+    if (has_blk) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float v[2];
-            asm("mov.b64 {%0, %1}, %2;" : "=f"(v[0]), "=f"(v[1]) : "l"(acc[i][j]));
-            acc[i][j] = 0ull;
+        for (int j = 0; j < 4; ++j) {
+          float v[2];
+          asm("mov.b64 {%0, %1}, %2;" : "=f"(v[0]), "=f"(v[1]) : "l"(acc[i][j]));
+          acc[i][j] = 0ull;
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              float* p = sS + (row0 + i) * K + col0 + 16 * (j >> 1) + 2 * (j & 1) + q;
-              *p = fresh && g == 0 ? v[q] : *p + v[q];
-            }
+          for (int q = 0; q < 2; ++q) {
+            float* p = sS + (row0 + i) * K + col0 + 16 * (j >> 1) + 2 * (j & 1) + q;
+            *p = fresh ? v[q] : *p + v[q];
           }
-      }
-      __syncthreads();
+        }
     }
     fresh = false;
   };
@@ -368,16 +364,22 @@ __global__ void __launch_bounds__(GM_T) gram_kernel(const float* H, long long n,
   }
   __pipeline_wait_prior(0);
   add_up();
+  __syncthreads();
+  const float* all = sm + 2 * GM_RS * K;
   for (int e = tid; e < k * k; e += GM_T) {
     const int r = e / k, c = e % k;
-    const float v = c <= r ? sS[r * K + c] : sS[c * K + r];
+    const float* p = all + (c <= r ? r * K + c : c * K + r);
+    float v = p[0];
+#pragma unroll
+    for (int g = 1; g < GR; ++g) v += p[g * K * K];
     if (v != 0.f) atomicAdd(out + e, v);
   }
 }
 
 template <int KB>
 int launch_gram(const float* H, long long n, int k, float* out, cudaStream_t stream) {
-  const size_t smem = (2 * (size_t)GM_RS * 16 * KB + 256 * (size_t)KB * KB) * sizeof(float);
+  constexpr int B = KB / 2, GR = 10 / (B * (B + 1) / 2);          // as in the kernel
+  const size_t smem = (2 * (size_t)GM_RS * 16 * KB + GR * 256 * (size_t)KB * KB) * sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(gram_kernel<KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   const long long need = (n + 63) / 64;            // every block's sums are one more addition per entry
