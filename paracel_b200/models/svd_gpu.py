@@ -77,7 +77,9 @@ class SvdGpu(paralg):
         self.m = self.row_ptr.numel() - 1
         first, last = (int(self.row_ptr[0].item()), int(self.row_ptr[-1].item())) if self.m > 0 else (0, 0)
         self.t_ptr = self.t_rows = self.t_vals = None
-        free = torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
+        free = 1 << 29                    # small matrices do without asking, which takes 0.2 ms
+        if not _transpose_fits(last - first, self.N, free):
+            free = torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
         if not _transpose_fits(last - first, self.N, free):
             return
         # A^T in the same form: its products then add up in registers.  Scattering an entry at a time
@@ -85,10 +87,9 @@ class SvdGpu(paralg):
         # K = 32, against 0.14 ms for A H.
         c, order = torch.sort(self.cols[first:last], stable=True)
         row_of = torch.repeat_interleave(torch.arange(self.m, device=dev, dtype=torch.int32),
-                                         self.row_ptr[1:] - self.row_ptr[:-1])
+                                         self.row_ptr[1:] - self.row_ptr[:-1], output_size=last - first)
         self.t_rows, self.t_vals = row_of[order], self.vals[first:last][order]
-        self.t_ptr = torch.zeros(self.N + 1, dtype=torch.int64, device=dev)
-        self.t_ptr[1:] = torch.cumsum(torch.bincount(c, minlength=self.N), 0)
+        self.t_ptr = torch.searchsorted(c, torch.arange(self.N + 1, device=dev, dtype=torch.int32))
 
     def _times_transposed(self, W: torch.Tensor, out: torch.Tensor) -> None:
         """``out = A^T W`` for this rank's rows."""
