@@ -82,9 +82,12 @@ class PageRankGpu(paralg):
         self.rank_local = torch.where(self.has_out, torch.full_like(od, init), torch.zeros_like(od))
         self.rank_new = torch.empty_like(self.rank_local)
         self.acc = torch.zeros(max(self.n_local, 1), device=dev)
-        # On small graphs the kernel that reads the sums clears them, which saves a launch (20 iterations on
-        # 2^14 vertices: 435 -> 411 us; on 2^17: 529 -> 517 us).  From 2^18 on a memset of its own is faster
-        # (2^18: 693 -> 625 us, 2^22: 6.6 -> 3.8 ms).
+        # On small graphs the kernel that reads the sums clears them, which saves a launch; on larger ones its
+        # stores cost more than a memset of their own.  20 iterations on R-MAT graphs with 3, 6, 16 and 24
+        # edges a vertex, memset against cleared by the reader: 2^14 vertices 491 / 468 / 432 / 425 against
+        # 466 / 445 / 399 / 404 us, 2^17 547 / 588 / 587 / 633 against 528 / 571 / 571 / 619, 2^18 630 / 663 / 736 /
+        # 802 against 676 / 723 / 789 / 863, 2^22 2.5 / 3.2 / 6.0 / 8.5 against 5.2 / 6.0 / 8.8 / 11.4 ms: the line is
+        # the same for all four.  Why the stores cost that much above it is not known.
         self.acc_clean = self.n_local <= 1 << 17
         self.plan = self._choose_plan()
         # contribution table for iteration 0 lives in tables[0]

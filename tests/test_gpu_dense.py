@@ -290,3 +290,32 @@ def test_sparse_gradient_read_one_step_ahead(n, F, logistic, valued):
         # half a unit of the fixed-point table per term; margins of up to 70 terms; fp32 sums of cnt terms
         bound = (cnt * 2.0 ** -15 if logistic else 0) + (cnt + 90) * 2.0 ** -23 * mag
         assert bool(((grad.double() - ref).abs() <= bound + 1e-30).all())
+
+
+@pytest.mark.parametrize("cap", [2048, 4096])
+@pytest.mark.parametrize("clean", [True, False])
+def test_pagerank_of_a_graph_with_more_rows_than_links_in_a_block(monkeypatch, cap, clean):
+    """Blocks of 1500 to 3000 rows keep no row pointers; rows are cut by block ends, one spans several blocks.
+    Several steps with both ways of clearing the sums, each published by the step's last block."""
+    from paracel_b200.models.pagerank_gpu import PageRankGpu
+    monkeypatch.setenv("PCL_PAGERANK_CAP", str(cap))
+    g = torch.Generator(device="cuda").manual_seed(cap)
+    n, steps = 200_000, 6
+    src = torch.randint(0, n, (270_000,), device="cuda", generator=g)
+    dst = torch.randint(0, n, (270_000,), device="cuda", generator=g)
+    dst[:9000] = 77_777
+    m = PageRankGpu(n, 0.85, device="cuda")
+    m.load_edges(src, dst)
+    m.acc_clean = clean
+    od = torch.bincount(src, minlength=n).double()
+    r = (od > 0).double() / float((od > 0).sum())
+    inv = torch.where(od > 0, 1 / od, torch.zeros_like(od))
+    for _ in range(steps):
+        m.step()
+        r = 0.15 + 0.85 * torch.zeros_like(r).index_add_(0, dst, (r * inv)[src])
+    # positive terms, chains of at most 128 additions (a thread's or a lane's share, a warp's tree, the blocks)
+    assert bool(((m.ranks().double() - r).abs() <= steps * (128 + 8) * 2.0 ** -24 * r).all())
+    m.paracel_sync()
+    m.paracel_check()
+    assert not clean or not bool(m.acc.any())
+    m.free()
