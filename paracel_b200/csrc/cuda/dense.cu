@@ -83,7 +83,7 @@ struct BupArgs {
   int handler;
   float lr, lambda;
   const long long* ready;       // local flag array the peers publish "delta ready" into
-  long long* const* ready_ptrs; // world pointers to every rank's "ready" array (null: published before)
+  long long* const* ready_ptrs; // world pointers to every rank's "ready" array
   long long epoch;
   unsigned long long timeout_ns;
   PclStatus* status;
@@ -113,7 +113,7 @@ template <bool IS_MAX>
 __global__ void __launch_bounds__(256) dense_bupdate_kernel(BupArgs a) {
   __shared__ int ok;
   // This rank's own "ready": the first block stores it, and waits for nobody before that.
-  if (a.ready_ptrs != nullptr && blockIdx.x == 0 && threadIdx.x == 0)
+  if (blockIdx.x == 0 && threadIdx.x == 0)
     pcl_publish(a.ready_ptrs, a.world, a.rank, a.epoch);
   // a single rank's delta was written by earlier work of this stream: nobody to wait for
   const bool wait = a.world > 1 && a.ready != nullptr && a.epoch > 0;
@@ -279,6 +279,7 @@ PCL_API int pcl_dense_bupdate(float* theta, const float* const* deltas, long lon
                               unsigned long long timeout_ns, PclStatus* status, long long* const* done_ptrs,
                               unsigned int* block_counter, double* nnz_out, cudaStream_t stream) {
   if (L <= 0) return 0;
+  if (ready_ptrs == nullptr) return (int)cudaErrorInvalidValue;
   BupArgs a{theta, deltas, L, S, world, rank, handler, lr, lambda, ready, ready_ptrs, epoch, timeout_ns,
             status, done_ptrs, block_counter, nnz_out};
   long long blocks = (S / 4 + 255) / 256;
