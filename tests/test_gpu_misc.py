@@ -453,11 +453,13 @@ def test_kmeans_accumulate_on_both_sides_of_the_point_count_that_picks_its_sums(
 @pytest.mark.parametrize("k", [30, 64, 96, 128])
 def test_gram_chains_are_bounded(k):
     """2.5 M equal rows: a chain of one block's rows, all in one register, is off by 1.1e-4 at k > 64;
-    chains of 1280 terms and of the blocks' sums by half a unit per addition at most, 4.7e-5."""
+    chains of 1280 terms (for k <= 64 a group's share of the block) and of the groups' and blocks' sums by half a
+    unit per addition at most, 4.7e-5."""
     from paracel_b200.ops.misc import gram
     n, h = 2_500_000, 1.0 + 2.0 ** -10 + 2.0 ** -13
     G = gram(torch.full((n, k), h, device="cuda"))
-    chain = 1280 + n // (296 * 1280) + 10 + 296
+    rows = n // 296 + 1
+    chain = (1280 + rows // 1280 if k > 64 else rows // (10 if k <= 32 else 3) + 1) + 10 + 296
     assert float((G.double() / (n * h * h) - 1).abs().max()) <= chain * 2.0 ** -25
 
 
