@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(128) lda_loglik_rows_kernel(LlArgs a) {
   if (lane == 0 && acc != 0.0) atomicAdd(a.out, acc);
 }
 
-// any other K
+// Any other K, and tables off 16-byte boundaries.  The sampler takes neither; the entry point does.
 __global__ void __launch_bounds__(128) lda_loglik_kernel(LlArgs a) {
   const int lane = threadIdx.x & 31;
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;

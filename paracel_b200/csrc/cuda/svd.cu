@@ -233,9 +233,10 @@ int launch_spmm(const long long* row_ptr, const int* cols, const float* vals, lo
 // block of 256 threads takes 128 rows at a time: thread (ty, tx) owns rows ty + 16 i (i < 8) and columns
 // tx + 16 j, sums over even and odd components in the halves of packed multiply-adds.  P^T and, for
 // the second product, P stay in shared memory as rows of components, and the product of the first
-// takes the place of the rows there.  Bound by shared-memory passes: 32 + 4 KB a thread for 64 KB
-// multiply-adds over four components (400 k x 32 and 100 k x 32 twice: 55 us a call on average with 4
-// rows a thread and 4-byte loads of P).
+// takes the place of the rows there.  Bound by shared-memory passes: a thread loads 8 + KB times
+// 16 bytes for 32 KB multiply-adds over four components.  The products of the SVD, 400 k x 32 and
+// 100 k x 32 twice, take 83 and 29 us (86 and 31 with 4 rows a thread; at 400 k x 52 that form was faster, 199
+// against 211 us, at 400 k x 112 slower, 715 against 643).
 template <int KB, bool TWICE>
 __global__ void __launch_bounds__(256) rows_times_kernel(const float* __restrict__ M, long long n, int K,
                                                          const float* __restrict__ P, float* __restrict__ out) {

@@ -7,7 +7,7 @@ file it read to the owners); the users are partitioned over the ranks as by the 
 ``fmap`` pattern (als.hpp:174).  ``solve`` is
 
     H_local = paracel_read_multi(keys of the items my users rated)     sparse keyed pull over NVLink
-    W       = batched normal equations + Cholesky, one CTA per user    csrc/cuda/als.cu
+    W       = batched normal equations + Cholesky                      csrc/cuda/als.cu
     paracel_write_multi(keys of my users, W)                           rows W_<uid> to their owners
 
 so no rank ever holds all of H, unlike the host path, which streams the whole factor file
