@@ -49,12 +49,14 @@ def host_rand(shape, seed: int, device, scale: float = 1.0, shift: float = 0.0) 
     """``torch.rand(shape, generator=g) * scale + shift`` for a fresh CPU generator ``g`` with
     ``manual_seed(seed)``, made on the device (number for number where the scaled values are exact,
     as they are for 2 and -1)."""
-    g = torch.Generator()
-    g.manual_seed(seed)                        # refuses what the generator refuses
+    if type(seed) is not int or not 0 <= seed < 1 << 32:       # plain seeds need no generator, 10 us
+        g = torch.Generator()
+        g.manual_seed(seed)                    # refuses what the generator refuses, maps negative seeds
+        seed = g.initial_seed()
     if torch.device(device).type != "cuda":
         raise ValueError("the numbers are made on a CUDA device")
     out = torch.empty(shape, device=device, dtype=torch.float32)
-    _lib.call("pcl_mt19937_uniform", out, out.numel(), g.initial_seed() & 0xffffffff, float(scale), float(shift),
+    _lib.call("pcl_mt19937_uniform", out, out.numel(), seed & 0xffffffff, float(scale), float(shift),
               _lib.stream_ptr())
     return out
 
