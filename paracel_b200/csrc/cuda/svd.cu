@@ -22,7 +22,7 @@ namespace {
 // but half a millisecond, and used 8 of its 32 lanes.)  What is left is bound by the
 // gathers of 4 K bytes per entry out of L2: four are in flight per group before the first is used.
 // Rows of even length, against a warp per row: 500 k x 40 entries out of 20 k columns, K = 16 / 32 / 52 / 128,
-// 157 / 267 / 424 / 679 us against 672 / 674 / 676 / 691; 400 k x 16 out of 100 k 69 / 101 / 151 / 282 against
+// 157 / 267 / 423 / 679 us against 672 / 674 / 676 / 691; 400 k x 16 out of 100 k 69 / 101 / 175 / 282 against
 // 243 / 245 / 246 / 258.  Short rows with K > 64 and small matrices stay behind it (400 k x 5, K = 128, 150 us
 // against 128; 20 k x 15, K = 128, 27.6 against 20.6): more row ends per entry, and a chain of searches before
 // the first gather.
@@ -48,8 +48,9 @@ __device__ __forceinline__ long long row_of_entry(const long long* row_ptr, long
   return lo;
 }
 
-template <int G, bool TRANS>
-__global__ void __launch_bounds__(256, G >= 16 && !TRANS ? 5 : 0) spmm_kernel(const long long* __restrict__ row_ptr,
+// STRAIGHT: batches of four entries inside one row skip the questions about row ends.
+template <int G, bool TRANS, bool STRAIGHT>
+__global__ void __launch_bounds__(256, STRAIGHT ? 5 : 0) spmm_kernel(const long long* __restrict__ row_ptr,
                                                    const int* __restrict__ cols,
                                                    const float* __restrict__ vals, long long n_rows,
                                                    long long n_ent, int L, const float* __restrict__ X,
@@ -134,9 +135,7 @@ __global__ void __launch_bounds__(256, G >= 16 && !TRANS ? 5 : 0) spmm_kernel(co
     }
     float4 h[U];
     if constexpr (!TRANS) {
-      // all of the current row: without the questions below 889 -> 693 us on 100 k x 200 entries, K = 128; with
-      // narrow groups a warp would go both ways (400 k x 5, K = 32: 77 -> 83 us)
-      if (G >= 16 && p0 >= gs && p0 + U <= (end < ge ? end : ge)) {
+      if (STRAIGHT && p0 >= gs && p0 + U <= (end < ge ? end : ge)) {
 #pragma unroll
         for (int j = 0; j < U; ++j)
           h[j] = on ? __ldg(reinterpret_cast<const float4*>(X + (long long)c[j] * K + 4 * gl)) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -199,31 +198,42 @@ int launch_spmm(const long long* row_ptr, const int* cols, const float* vals, lo
                 long long n_ent, const float* X, int K, float* out, cudaStream_t stream) {
   int G = 1;
   while (4 * G < K) G *= 2;
-  // Entries per group.  Narrow groups: 128, fewer while the chip's groups (2048 threads on each of 148 SMs)
-  // would not all get a segment.  From K = 36 on four times as many if that leaves four segments each (fewer
-  // row searches: 20 M entries, K = 128, 724 us at 128 and 679 at 512), and fewer only for a third of
-  // the groups (300 k entries, K = 128: 27.6 us against 33.8).
+  // Entries per group: 128, fewer while the chip's groups (2048 threads on each of 148 SMs) would not all get a
+  // segment.  From K = 36 on four times as many if that leaves four segments each (fewer row searches: 20 M
+  // entries, K = 128, 724 us at 128 and 679 at 512), and fewer than 2 G only for a third of the groups (300 k
+  // entries, K = 128: 27.6 us against 33.8).
   const bool wide = G >= 16 && !TRANS;
   int L = wide ? 512 : 128;
   while (L > 128 && n_ent / L < 4 * 148LL * 2048 / G) L /= 2;
-  while (L > 16 && n_ent / L < 148LL * (wide ? 640 : 2048) / G) L /= 2;
+  while (L > (wide ? 2 * G : 16) && n_ent / L < 148LL * 2048 / G) L /= 2;
+  while (L > 16 && n_ent / L < 148LL * 640 / G) L /= 2;
   const long long blocks = (n_ent + (256 / G) * (long long)L - 1) / ((256 / G) * (long long)L);
   const long long clear = (n_rows + 255) / 256;
   if (blocks > 0x7fffffffLL || clear > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
   if constexpr (!TRANS) {
-    if (n_rows * K <= 1 << 20) {                   // up to 4 MB clearing all is 2 us faster
+    if (n_rows * K <= 1 << 22) {                   // up to 16 MB clearing all is up to 2 us faster
       const cudaError_t e = cudaMemsetAsync(out, 0, (size_t)n_rows * K * sizeof(float), stream);
       if (e != cudaSuccess) return (int)e;
     } else {
       spmm_clear_kernel<<<(int)clear, 256, 0, stream>>>(row_ptr, n_rows, n_ent, L, K, out);
     }
   }
-#define PCL_SPMM(GG)                                                                                     \
-  case GG:                                                                                               \
-    spmm_kernel<GG, TRANS><<<(int)blocks, 256, 0, stream>>>(row_ptr, cols, vals, n_rows, n_ent, L, X, K, out); \
-    break;
+  // Straight batches pay where a group is a warp (100 k rows x 200 entries, K = 128: 889 -> 693 us).  Where two groups
+  // share one, a warp goes both ways unless rows are long: 100 k rows of up to 80 entries, K = 52, 113 -> 102 us,
+  // of up to 30 entries 55 -> 59 us.  Narrower groups lose either way (400 k x 5, K = 32: 77 -> 83 us).
+  const bool straight = G == 16 && n_ent >= 32 * n_rows;
+#define PCL_SPMM(GG, ST)                                                                                       \
+  spmm_kernel<GG, TRANS, ST><<<(int)blocks, 256, 0, stream>>>(row_ptr, cols, vals, n_rows, n_ent, L, X, K, out)
   switch (G) {
-    PCL_SPMM(1) PCL_SPMM(2) PCL_SPMM(4) PCL_SPMM(8) PCL_SPMM(16) PCL_SPMM(32)
+    case 1: PCL_SPMM(1, false); break;
+    case 2: PCL_SPMM(2, false); break;
+    case 4: PCL_SPMM(4, false); break;
+    case 8: PCL_SPMM(8, false); break;
+    case 16:
+      if (straight) PCL_SPMM(16, !TRANS);
+      else PCL_SPMM(16, false);
+      break;
+    case 32: PCL_SPMM(32, !TRANS); break;
   }
 #undef PCL_SPMM
   return pcl_last_error();

@@ -463,9 +463,9 @@ def test_gram_chains_are_bounded(k):
     assert float((G.double() / (n * h * h) - 1).abs().max()) <= chain * 2.0 ** -25
 
 
-@pytest.mark.parametrize("n,per,K", [(9001, 130, 128), (40_003, 7, 32), (30_001, 16, 52), (120_001, 200, 128)])
+@pytest.mark.parametrize("n,per,K", [(33_001, 40, 128), (140_003, 7, 32), (90_001, 16, 52), (90_001, 50, 64), (120_001, 200, 128)])
 def test_csr_product_writes_every_row_of_a_dirty_output(n, per, K):
-    """Outputs beyond 4 MB are cleared by rows: those without entries and those cut by a segment's end
+    """Outputs beyond 16 MB are cleared by rows: those without entries and those cut by a segment's end
     (of 512 entries in the last case), while the others are stored once."""
     from paracel_b200.ops.svd import spmm_csr
     g = torch.Generator(device="cuda").manual_seed(n)
