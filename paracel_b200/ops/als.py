@@ -15,9 +15,9 @@ def _kpad(k: int) -> int:
 
 def als_solve(user_ptr: torch.Tensor, item_idx: torch.Tensor, rating: torch.Tensor, H: torch.Tensor,
               lam: float, seg_len: int = 4096) -> torch.Tensor:
-    """``user_ptr`` (int64, n_users + 1) delimits each user's entries of ``item_idx`` (int32 rows
-    of H) and ``rating`` (fp32).  Users with more than ``seg_len`` ratings are split over
-    several CTAs.  Returns W [n_users, k]."""
+    """``user_ptr`` (int64, n_users + 1, ascending) delimits each user's entries of ``item_idx`` (int32
+    rows of H) and ``rating`` (fp32), all on one device.  Users with more than ``seg_len`` ratings are split
+    over several CTAs.  Returns W [n_users, k]."""
     dev = H.device
     for name, t in (("user_ptr", user_ptr), ("item_idx", item_idx), ("rating", rating)):
         if t.device != dev:                   # their addresses go to the kernels as they are
